@@ -142,24 +142,18 @@ __global__ void cmpdt_kernel(const double* __restrict__ ud, const float* __restr
     long long oct = oct0 + cell_id / 8;
     int cell = (int)(cell_id % 8);
     const bool ref = refined ? refined[cell_id] != 0 : (refbits ? ((refbits[oct] >> cell) & 1) != 0 : false);
-    if (!ref && !fp32) {
-      const double* o = ud + oct * 40 + cell;
-      const double r = o[0], m1 = o[8], m2 = o[16], m3 = o[24], E = o[32];
-      m = r * vol;
-      ek = E * vol;
-      const double rm = r > C.smallr ? r : C.smallr;
-      ei = E * vol;
-      ei -= 0.5 * (m1 * m1) / rm * vol;
-      ei -= 0.5 * (m2 * m2) / rm * vol;
-      ei -= 0.5 * (m3 * m3) / rm * vol;
-      dt = cmpdt_cell(r, m1, m2, m3, E, C);
-    } else if (!ref) {
-      // an FP32-bulk cell in the fused epilogue's FP32-bulk form, so that a
-      // level's values do not depend on which of the two computed them
-      const float* o = uf + oct * kBulkF + cell;
+    if (!ref) {
+      // in the fused epilogue's form, so that a level's values do not depend
+      // on which of the two computed them
       CflAcc a;
-      a.add_bulk(o[0], o[8], o[16], o[24], ud[oct * kBulkD + cell], C);
-      a.scale_bulk(vol);
+      if (!fp32) {
+        const double* o = ud + oct * 40 + cell;
+        a.add(o[0], o[8], o[16], o[24], o[32], C);
+      } else {
+        const float* o = uf + oct * kBulkF + cell;
+        a.add(o[0], o[8], o[16], o[24], ud[oct * kBulkD + cell], C);
+      }
+      a.scale(vol);
       m = a.mass;
       ek = a.ekin;
       ei = a.eint;
@@ -991,10 +985,11 @@ __global__ void __launch_bounds__(kGatherThreads)
       const int2 fa = fathers[gg];
       if (fa.x >= 0 && !((refmask[fa.x] >> fa.y) & 1u)) {
         const double* q = cell[threadIdx.x];
-        acc.add(q[0], q[1], q[2], q[3], q[4], C, vol);
+        acc.add(q[0], q[1], q[2], q[3], q[4], C);
       }
     }
   }
+  acc.scale(vol);
   cfl_block_reduce<kGatherThreads / 32>(acc, C, red, partial + (size_t)blockIdx.x * 5);
 }
 
@@ -1034,11 +1029,11 @@ __global__ void __launch_bounds__(kGatherThreads)
       const int2 fa = fathers[gg];
       if (fa.x >= 0 && !((refmask[fa.x] >> fa.y) & 1u)) {
         const double* q = cell[threadIdx.x];
-        acc.add_bulk((float)q[0], (float)q[1], (float)q[2], (float)q[3], q[4], C);
+        acc.add(q[0], q[1], q[2], q[3], q[4], C);
       }
     }
   }
-  acc.scale_bulk(vol);
+  acc.scale(vol);
   cfl_block_reduce<kGatherThreads / 32>(acc, C, red, partial + (size_t)blockIdx.x * 5);
 }
 

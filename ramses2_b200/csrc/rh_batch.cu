@@ -153,11 +153,11 @@ __global__ void batch_cfl_kernel(BatchProb P, const double* ud, const float* uf,
     if (!fp32) {
       const double* p = ud + o * 40 + cell;
       acc.add(p[0], p[8], p[16], p[24], p[32], A);
-    } else {  // the FP32-bulk form the fused epilogue of the problem's steps uses
+    } else {
       const float* p = uf + o * kBulkF + cell;
-      acc.add_bulk(p[0], p[8], p[16], p[24], ud[o * kBulkD + cell], A);
-      acc.scale_bulk(A.vol);
+      acc.add(p[0], p[8], p[16], p[24], ud[o * kBulkD + cell], A);
     }
+    acc.scale(A.vol);
   }
   double v[4] = {acc.mass, acc.ekin, acc.eint, acc.dt(A.cfl)};
   for (int off = 16; off > 0; off >>= 1) {

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(Geo<T, V, TXO, TYO>::NT, MINB) batch_step_kern
         if (g && !(sizeof(T) == 4 && 2 * TXO + 2 == 16)) __syncthreads();
         batch_plane<T, TXO, TYO, SLOPE, RIEMANN>(g, &acc);
       }
-      if constexpr (sizeof(T) == 4) acc.scale_bulk(rh_bA.vol);
+      acc.scale(rh_bA.vol);
       cfl_block_reduce<G::NWARP>(acc, rh_bA.cfl, reinterpret_cast<double*>(rh_smem + G::oRed), rh_b_out);
       continue;
     }

@@ -178,10 +178,10 @@ template <typename T, int RIEMANN> __device__ __forceinline__ void riemann(const
 }
 
 // ---------------------------------------------------------------------------
-// CFL time step of one cell from conserved FP64 values, cmpdt
-// (godunov_utils.f90:228-333) with bb=0, induction=.false.  With zero
-// magnetic field the reference's fast speed sqrt(c2+sqrt(c2**2)) equals
-// sqrt(a2) exactly in IEEE arithmetic (sqrt(fl(x*x)) == x).
+// Constants of cmpdt (godunov_utils.f90:228-333) with bb=0,
+// induction=.false.  With zero magnetic field the reference's fast speed
+// sqrt(c2+sqrt(c2**2)) equals sqrt(a2) exactly in IEEE arithmetic
+// (sqrt(fl(x*x)) == x).
 // ---------------------------------------------------------------------------
 struct CflConst {
   double gamma, gm1, smallr, smallp;  // smallp = smallc**2/gamma
@@ -192,33 +192,6 @@ struct CflConst {
   double k0;                          // 2*courant*dx/(1+sqrt(1+2*courant*1e-4)): dt*ctot without gravity
   int ndim;
 };
-
-__device__ __forceinline__ double cmpdt_cell(double r, double mx, double my, double mz, double E,
-                                             const CflConst& C) {
-  r = r > C.smallr ? r : C.smallr;
-  double ir = 1.0 / r;
-  double u = mx * ir, v = my * ir, w = mz * ir;
-  double e = E - 0.5 * r * (u * u);
-  e = e - 0.5 * r * (v * v);
-  e = e - 0.5 * r * (w * w);
-  double p = C.gm1 * e;
-  double pf = r * C.smallp;
-  p = p > pf ? p : pf;
-  double c = sqrt(C.gamma * p * ir);
-  double ctot = fabs(u) + c;
-  if (C.ndim > 1) ctot += fabs(v) + c;
-  if (C.ndim > 2) ctot += fabs(w) + c;
-  double dtcell;
-  if (C.gsum_dx == 0.0) {
-    // grav = max(0, 1e-4): the square root is a constant of the launch
-    dtcell = C.k0 / ctot;
-  } else {
-    double grav = C.gsum_dx / (ctot * ctot);
-    grav = grav > 0.0001 ? grav : 0.0001;
-    dtcell = C.two_cdx / (ctot * (1.0 + sqrt(1.0 + C.two_c * grav)));
-  }
-  return dtcell < C.cdx_smallc ? dtcell : C.cdx_smallc;
-}
 
 // ---------------------------------------------------------------------------
 // PTX helpers: mbarrier + bulk async copy (global -> shared, no multicast)

@@ -208,55 +208,23 @@ template <typename T> struct StateArgs {
 
 constexpr long long kWaitBound = 1ll << 22;  // bounded mbarrier spin (seconds at most)
 
-// Per-thread FP64 CFL / conserved-total accumulation of one new cell
-// (courant_fine.f90:317-386 + cmpdt).
-// Per-thread courant_fine accumulators.  The cell time step of cmpdt
-// (godunov_utils.f90:228-333) is a decreasing function of the cell's summed
-// signal speed ctot (dx-scaled constant over ctot, or its gravity form), so
-// the thread keeps the largest ctot and converts it once: min over cells of
-// dt(ctot) = dt(max ctot), with no division or square root of the dt formula
-// per cell.
+// Per-thread courant_fine accumulators (courant_fine.f90:317-386 + cmpdt).
+// The cell time step of cmpdt (godunov_utils.f90:228-333) is a decreasing
+// function of the cell's summed signal speed ctot (dx-scaled constant over
+// ctot, or its gravity form), so the thread keeps the largest ctot and
+// converts it once: min over cells of dt(ctot) = dt(max ctot), with no
+// division or square root of the dt formula per cell.  The three sums stay
+// unscaled until scale() multiplies them by the cell volume once, the kinetic
+// energy is (m1^2 + m2^2 + m3^2) / (2 rho) and ctot = (|m1| + |m2| + |m3|) /
+// rho + ndim c: about 30 FP64 operations a cell, where squaring the
+// velocities and scaling each term by the volume took about 60.
 struct CflAcc {
   double mass = 0, ekin = 0, eint = 0, cmax = 0;
   __device__ __forceinline__ void add(double r, double m1, double m2, double m3, double E, const LevelArgs& A) {
-    add(r, m1, m2, m3, E, A.cfl, A.vol);
+    add(r, m1, m2, m3, E, A.cfl);
   }
-  __device__ __forceinline__ void add(double r, double m1, double m2, double m3, double E, const CflConst& C,
-                                      double vol) {
-    mass += r * vol;
-    ekin += E * vol;
-    const double rm = r > C.smallr ? r : C.smallr;
-    const double irm = vrcp(rm);
-    double ei = E * vol;
-    ei -= 0.5 * (m1 * m1) * irm * vol;
-    ei -= 0.5 * (m2 * m2) * irm * vol;
-    ei -= 0.5 * (m3 * m3) * irm * vol;
-    eint += ei;
-    const double u = m1 * irm, v = m2 * irm, w = m3 * irm;
-    double e = E - 0.5 * rm * (u * u);
-    e = e - 0.5 * rm * (v * v);
-    e = e - 0.5 * rm * (w * w);
-    double p = C.gm1 * e;
-    const double pf = rm * C.smallp;
-    p = p > pf ? p : pf;
-    const double c = vsqrt(C.gamma * p * irm);
-    double ctot = fabs(u) + c;
-    if (C.ndim > 1) ctot += fabs(v) + c;
-    if (C.ndim > 2) ctot += fabs(w) + c;
-    cmax = ctot > cmax ? ctot : cmax;
-  }
-  // The same quantities for an FP32-bulk cell (density and momenta held in
-  // FP32, E in FP64), in fewer FP64 operations: the three sums stay unscaled
-  // until scale_bulk multiplies them by the cell volume once, the kinetic
-  // energy is (m1^2 + m2^2 + m3^2) / (2 rho) (the squares of FP32 momenta
-  // are exact in FP64) and ctot = (|m1| + |m2| + |m3|) / rho + ndim c.
-  __device__ __forceinline__ void add_bulk(float rf, float m1f, float m2f, float m3f, double E,
-                                           const LevelArgs& A) {
-    add_bulk(rf, m1f, m2f, m3f, E, A.cfl);
-  }
-  __device__ __forceinline__ void add_bulk(float rf, float m1f, float m2f, float m3f, double E,
-                                           const CflConst& C) {
-    const double r = rf, m1 = m1f, m2 = m2f, m3 = m3f;
+  // (an FP32-bulk cell's density and momenta widen exactly)
+  __device__ __forceinline__ void add(double r, double m1, double m2, double m3, double E, const CflConst& C) {
     mass += r;
     ekin += E;
     const double rm = r > C.smallr ? r : C.smallr;
@@ -273,7 +241,7 @@ struct CflAcc {
     const double ctot = fma(a, irm, (double)C.ndim * c);
     cmax = ctot > cmax ? ctot : cmax;
   }
-  __device__ __forceinline__ void scale_bulk(double vol) {
+  __device__ __forceinline__ void scale(double vol) {
     mass *= vol;
     ekin *= vol;
     eint *= vol;
@@ -472,15 +440,14 @@ __device__ __forceinline__ void ctoprim_f64(const double* sd, int cell, bool fx,
   U[0] = d; U[1] = mx; U[2] = my; U[3] = mz; U[4] = E;
   const double r = d > H.smallr ? d : H.smallr;
   ir = vrcp(r);
-  const double u = mx * ir, v = my * ir, w = mz * ir;
-  const double ekin = (0.5 * r) * fma(u, u, fma(v, v, w * w));
-  double eint = E - ekin;
+  // eint = E - |m|^2 / (2 rho), the velocities with the predictor's gravity
+  double eint = fma(-0.5 * ir, fma(mx, mx, fma(my, my, mz * mz)), E);
   const double emin = H.smalle * r;
   eint = eint > emin ? eint : emin;
   q[0] = r;
-  q[1] = u + H.grav[0];
-  q[2] = v + H.grav[1];
-  q[3] = w + H.grav[2];
+  q[1] = fma(mx, ir, H.grav[0]);
+  q[2] = fma(my, ir, H.grav[1]);
+  q[3] = fma(mz, ir, H.grav[2]);
   q[4] = H.gm1 * eint;
 }
 

@@ -92,15 +92,18 @@ __device__ __forceinline__ double half_momentum_bound(double dq, double rm1, dou
   return vcopysign(vmin(vabs(dq), dlim), dq);
 }
 
-// HLLC (Toro), godunov_utils.f90:638-852.  q = (rho, un, ut1, ut2, p);
-// f = (mass, normal momentum, t1 momentum, t2 momentum, total energy).
+// HLLC (Toro), godunov_utils.f90:638-852, times dt/dx.  q = (rho, un, ut1,
+// ut2, p); f = (mass, normal momentum, t1 momentum, t2 momentum, total
+// energy).  The side's total energy is formed after the side is chosen (the
+// reference forms both and takes one), and dt/dx enters once through the
+// sampled velocity and pressure instead of scaling the five fluxes: with the
+// shorter reciprocals and square roots 78 FP64-pipe operations a face, 104
+// before.
 template <class V> __device__ __forceinline__ void riemann_hllc(const V* ql, const V* qr, V* f, const HydroK<V>& H) {
   const V rl = vmax(ql[0], H.smallr), ul = ql[1], vl = ql[2], wl = ql[3];
   const V Pl = vmax(ql[4], rl * H.smallp_riem);
   const V rr = vmax(qr[0], H.smallr), ur = qr[1], vr = qr[2], wr = qr[3];
   const V Pr = vmax(qr[4], rr * H.smallp_riem);
-  const V etotl = vfma(Pl, H.entho, H.half * rl * vfma(ul, ul, vfma(vl, vl, wl * wl)));
-  const V etotr = vfma(Pr, H.entho, H.half * rr * vfma(ur, ur, vfma(vr, vr, wr * wr)));
   const V cfl = vsqrt(vmax(H.gamma * Pl * vrcp(rl), H.smallc2));
   const V cfr = vsqrt(vmax(H.gamma * Pr * vrcp(rr), H.smallc2));
   const V cmx = vmax(cfl, cfr);
@@ -116,19 +119,21 @@ template <class V> __device__ __forceinline__ void riemann_hllc(const V* ql, con
   const auto left = mor(slpos, vgt(ustar, H.zero));
   const auto star = mor(mand(left, mnot(slpos)), mand(mnot(left), vgt(SR, H.zero)));
   const V rs = vsel(left, rl, rr), us = vsel(left, ul, ur), vs = vsel(left, vl, vr), ws = vsel(left, wl, wr);
-  const V Ps = vsel(left, Pl, Pr), Es = vsel(left, etotl, etotr), Ss = vsel(left, SL, SR);
+  const V Ps = vsel(left, Pl, Pr), Ss = vsel(left, SL, SR);
+  const V Es = vfma(Ps, H.entho, H.half * rs * vfma(us, us, vfma(vs, vs, ws * ws)));
   const V sdu = Ss - us;
   const V id = vrcp(Ss - ustar);
   const V ro = vsel(star, rs * sdu * id, rs);
   const V uo = vsel(star, ustar, us);
   const V Po = vsel(star, Pstar, Ps);
   const V Eo = vsel(star, vfma(sdu, Es, vfma(Pstar, ustar, -(Ps * us))) * id, Es);
-  const V mu = ro * uo;
+  const V uc = uo * H.dtdx;
+  const V mu = ro * uc;
   f[0] = mu;
-  f[1] = vfma(mu, uo, Po);
+  f[1] = vfma(mu, uo, Po * H.dtdx);
   f[2] = mu * vs;
   f[3] = mu * ws;
-  f[4] = (Eo + Po) * uo;
+  f[4] = (Eo + Po) * uc;
 }
 
 // Conservative state and physical flux of a rotated primitive state.
@@ -183,9 +188,12 @@ template <class V> __device__ __forceinline__ void riemann_hll(const V* ql, cons
 
 template <class V, int RIEMANN> __device__ __forceinline__ void riemann_dtdx(const V* ql, const V* qr, V* f,
                                                                             const HydroK<V>& H) {
+  if (RIEMANN == 3) {
+    riemann_hllc(ql, qr, f, H);
+    return;
+  }
   if (RIEMANN == 1) riemann_llf(ql, qr, f, H);
-  else if (RIEMANN == 2) riemann_hll(ql, qr, f, H);
-  else riemann_hllc(ql, qr, f, H);
+  else riemann_hll(ql, qr, f, H);
 #pragma unroll
   for (int n = 0; n < 5; ++n) f[n] = f[n] * H.dtdx;
 }
