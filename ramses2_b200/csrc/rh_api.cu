@@ -1178,7 +1178,7 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
     H.smallp_trace = smallr * (smallc * smallc);
     H.smallp_riem = smallc * smallc / gamma;
     H.smax_cap = smax_cap; H.dtdx = dt / dx;
-    H.zero = 0.0; H.half = 0.5; H.two = 2.0;
+    H.zero = 0.0; H.quarter = 0.25; H.half = 0.5; H.two = 2.0;
     H.gm1 = gamma - 1.0; H.smalle = A.smalle_d;
     for (int d = 0; d < 3; ++d) H.grav[d] = gh[d];
     RH_CUDA(fn(A, &S, &H, nblocks, st));
@@ -1191,7 +1191,7 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
     H.smallp_trace = b(smallr * (smallc * smallc));
     H.smallp_riem = b(smallc * smallc / gamma);
     H.smax_cap = b(std::min(smax_cap, 3.0e38)); H.dtdx = b(dt / dx);
-    H.zero = b(0.0); H.half = b(0.5); H.two = b(2.0);
+    H.zero = b(0.0); H.quarter = b(0.25); H.half = b(0.5); H.two = b(2.0);
     H.gm1 = b(gamma - 1.0); H.smalle = b(A.smalle_d);
     for (int d = 0; d < 3; ++d) H.grav[d] = b(gh[d]);
     RH_CUDA(fn(A, &S, &H, nblocks, st));

@@ -110,6 +110,7 @@ template <class V> __device__ __forceinline__ void batch_hydro(const BatchProb& 
   H.smax_cap = b(sizeof(typename Lane<V>::S) == 4 && cap > 3.0e38 ? 3.0e38 : cap);
   H.dtdx = b(dt / P.dx);
   H.zero = b(0.0);
+  H.quarter = b(0.25);
   H.half = b(0.5);
   H.two = b(2.0);
   H.gm1 = b(P.gamma - 1.0);

@@ -19,26 +19,10 @@ template <class V> struct HydroK {
   V smallp_riem;   // smallc**2/gamma             (godunov_utils.f90:363,511,676)
   V smax_cap;      // courant*dx/dt               (umuscl.f90:99)
   V dtdx;
-  V zero, half, two;
+  V zero, quarter, half, two;
   V gm1, smalle;   // gamma-1, smallc**2/gamma/(gamma-1) (umuscl.f90:1778)
   V grav[3];       // constant_gravity*dt/2 (ctoprim predictor)
 };
-
-// TVD slope of one variable along one direction.
-template <class V, int SLOPE> __device__ __forceinline__ V limited_slope(V qm1, V q0, V qp1, const HydroK<V>& H) {
-  if (SLOPE == 0) return H.zero;
-  const V a = q0 - qm1, b = qp1 - q0;
-  if (SLOPE == 1) {  // minmod: 0 if a*b<=0, else the smaller-magnitude one
-    const V r = vsel(vgt(a, H.zero), vmin(a, b), vmax(a, b));
-    return vsel(vgt(a * b, H.zero), r, H.zero);
-  }
-  // moncen: dlft=2a, drgt=2b, dcen=(a+b)/2, dq=sign(dcen)*min(dlim,|dcen|),
-  // dlim = min(|dlft|,|drgt|) when dlft*drgt>0 else 0
-  const V dcen = H.half * (a + b);
-  const V slop = H.two * vmin(vabs(a), vabs(b));
-  const V dlim = vsel(vgt(a * b, H.zero), slop, H.zero);
-  return vcopysign(vmin(dlim, vabs(dcen)), dcen);
-}
 
 // slope_type 3, the positivity-preserving 3D unsplit slope (umuscl.f90:
 // 2207-2269): the central differences of a variable, scaled by
@@ -67,29 +51,72 @@ template <class V> __device__ __forceinline__ V momentum_bound(V dq, V rm1, V vm
 }
 
 
-// Half of limited_slope and of the momentum bound (FP64 lanes), for slope
-// types 1 and 2: bitwise 0.5 * the full values (scaling by two commutes with
-// rounding, so 0.5 * (2 min) = min and 0.5 * (0.5 (a + b)) = 0.25 (a + b)
-// exactly).  The FP64 body takes these: two multiplications fewer per slope,
-// and its registers fit without spilling (the FP32-bulk body ran 2 % slower
-// with them and keeps the full slopes times one half).
-template <int SLOPE> __device__ __forceinline__ double half_slope(double qm1, double q0, double qp1) {
+// Half of limited_slope and of the momentum bound, for slope types 0-2, as
+// the predictor takes them.  Half the moncen slope is the minmod of a, b and
+// (a + b)/4 (scaling by two commutes with rounding, so min(2|a|, 2|b|,
+// |a + b|/2)/2 is formed without the factors of two), half the minmod slope
+// half of that of a and b.
+// FP64: every compare, min or max of doubles is a DSETP on the FP64 pipe and
+// two FSELs, so the signs are compared as integers (no product a b, whose
+// underflow the reference's test a b > 0 would see), the smaller difference
+// is taken with its sign (no copysign) and two DSETPs remain of three.
+__device__ __forceinline__ bool same_sign(double a, double b) { return (__double2hiint(a) ^ __double2hiint(b)) >= 0; }
+template <int SLOPE>
+__device__ __forceinline__ double half_slope(double qm1, double q0, double qp1, const HydroK<double>&) {
   if (SLOPE == 0) return 0.0;
   const double a = q0 - qm1, b = qp1 - q0;
-  if (SLOPE == 1) {
-    const double r = vsel(vgt(a, 0.0), vmin(a, b), vmax(a, b));
-    return 0.5 * vsel(vgt(a * b, 0.0), r, 0.0);
-  }
-  const double dcen = 0.25 * (a + b);
-  const double dlim = vsel(vgt(a * b, 0.0), vmin(vabs(a), vabs(b)), 0.0);
-  return vcopysign(vmin(dlim, vabs(dcen)), dcen);
+  const double s = vabs(a) < vabs(b) ? a : b;
+  const double c = SLOPE == 1 ? 0.5 * s : 0.25 * (a + b);
+  const double m = SLOPE == 1 || vabs(c) < vabs(s) ? c : s;
+  return same_sign(a, b) ? m : 0.0;
 }
 __device__ __forceinline__ double half_momentum_bound(double dq, double rm1, double vm1, double v0, double rp1,
-                                                      double vp1, double ir0) {
+                                                      double vp1, double ir0, const HydroK<double>&) {
   const double dlft = rm1 * vabs(v0 - vm1);
   const double drgt = rp1 * vabs(vp1 - v0);
   const double dlim = vmin(dlft, drgt) * ir0;
   return vcopysign(vmin(vabs(dq), dlim), dq);
+}
+// FP32 lanes: minmod as max(min3, min(max3, 0)): the smallest when all are
+// positive, the largest when all are negative, else 0; four min/max a lane,
+// without compares, selects and copysign.
+template <int SLOPE>
+__device__ __forceinline__ float2 half_slope(float2 qm1, float2 q0, float2 qp1, const HydroK<float2>& H) {
+  if (SLOPE == 0) return H.zero;
+  const float2 a = q0 - qm1, b = qp1 - q0;
+  if (SLOPE == 1) return H.half * vmax(vmin(a, b), vmin(vmax(a, b), H.zero));
+  const float2 c = H.quarter * (a + b);
+  return vmax(vmin3(a, b, c), vmin(vmax3(a, b, c), H.zero));
+}
+__device__ __forceinline__ float2 half_momentum_bound(float2 dq, float2 rm1, float2 vm1, float2 v0, float2 rp1,
+                                                      float2 vp1, float2 ir0, const HydroK<float2>&) {
+  const float2 dlft = rm1 * vabs(v0 - vm1);
+  const float2 drgt = rp1 * vabs(vp1 - v0);
+  const float2 dlim = vmin(dlft, drgt) * ir0;
+  return vmax(vmin(dq, dlim), -dlim);
+}
+
+// Whether the predictor's floors (umuscl.f90:1059-1234) act on some interface
+// state of the cell: pr -+ d[a] of the density or the pressure below its
+// floor.  They rarely do, so the twelve compares and selects of a lane are
+// behind this test.  FP32: the lowest state of a variable is pr - max |d[a]|.
+// FP64: the sign-magnitude high words order like the numbers; a high word
+// not above the floor's may be a state below it (the selects then compare
+// exactly).
+__device__ __forceinline__ bool any_floor(const double (*qm)[5], const double (*qp)[5], const double*,
+                                          double (*)[5], const HydroK<double>& H) {
+  auto low = [&](int n) {
+    int m = __vimin3_s32(__double2hiint(qm[0][n]), __double2hiint(qm[1][n]), __double2hiint(qm[2][n]));
+    m = __vimin3_s32(m, __double2hiint(qp[0][n]), __double2hiint(qp[1][n]));
+    return min(m, __double2hiint(qp[2][n]));
+  };
+  return low(0) <= __double2hiint(H.smallr) || low(4) <= __double2hiint(H.smallp_trace);
+}
+__device__ __forceinline__ bool any_floor(const float2 (*)[5], const float2 (*)[5], const float2* pr,
+                                          float2 (*d)[5], const HydroK<float2>& H) {
+  const float2 lr = pr[0] - vmax3(vabs(d[0][0]), vabs(d[1][0]), vabs(d[2][0]));
+  const float2 lp = pr[4] - vmax3(vabs(d[0][4]), vabs(d[1][4]), vabs(d[2][4]));
+  return many(mor(vlt(lr, H.smallr), vlt(lp, H.smallp_trace)));
 }
 
 // HLLC (Toro), godunov_utils.f90:638-852, times dt/dx.  q = (rho, un, ut1,
@@ -220,10 +247,15 @@ template <class V> __device__ __forceinline__ void trace_cell(const V* q, V ir, 
       qp[a][n] = pr[n] - d[a][n];
       qm[a][n] = pr[n] + d[a][n];
     }
-    qp[a][0] = vsel(vlt(qp[a][0], H.smallr), r, qp[a][0]);
-    qp[a][4] = vsel(vlt(qp[a][4], H.smallp_trace), p, qp[a][4]);
-    qm[a][0] = vsel(vlt(qm[a][0], H.smallr), r, qm[a][0]);
-    qm[a][4] = vsel(vlt(qm[a][4], H.smallp_trace), p, qm[a][4]);
+  }
+  if (any_floor(qm, qp, pr, d, H)) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      qp[a][0] = vsel(vlt(qp[a][0], H.smallr), r, qp[a][0]);
+      qp[a][4] = vsel(vlt(qp[a][4], H.smallp_trace), p, qp[a][4]);
+      qm[a][0] = vsel(vlt(qm[a][0], H.smallr), r, qm[a][0]);
+      qm[a][4] = vsel(vlt(qm[a][4], H.smallp_trace), p, qm[a][4]);
+    }
   }
 }
 

@@ -128,18 +128,14 @@ __device__ __forceinline__ void plane2d_body(const LevelArgs& A, const StateArgs
     V d[3][5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      d[0][n] = limited_slope<V, SLOPE>(xm[n], cur[n], xp[n], H);
-      d[1][n] = limited_slope<V, SLOPE>(ym[n], cur[n], yp[n], H);
+      d[0][n] = half_slope<SLOPE>(xm[n], cur[n], xp[n], H);
+      d[1][n] = half_slope<SLOPE>(ym[n], cur[n], yp[n], H);
       d[2][n] = H.zero;
     }
     if (SLOPE > 0) {
-      d[0][1] = momentum_bound(d[0][1], xm[0], xm[1], cur[1], xp[0], xp[1], irc, H);
-      d[1][2] = momentum_bound(d[1][2], ym[0], ym[2], cur[2], yp[0], yp[2], irc, H);
+      d[0][1] = half_momentum_bound(d[0][1], xm[0], xm[1], cur[1], xp[0], xp[1], irc, H);
+      d[1][2] = half_momentum_bound(d[1][2], ym[0], ym[2], cur[2], yp[0], yp[2], irc, H);
     }
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int n = 0; n < 5; ++n) d[a][n] = H.half * d[a][n];
     V qm[3][5], qp[3][5];
     trace_cell(cur, irc, d, qm, qp, H);
 #pragma unroll

@@ -76,6 +76,23 @@ __device__ __forceinline__ float2 vsub_nc(float2 a, float2 b) {
 // the results differ from a compare-and-select at most in the sign of a zero.
 __device__ __forceinline__ float2 vmin(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 __device__ __forceinline__ float2 vmax(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+// three-operand forms (one instruction a lane on sm_100)
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float2 vmin3(float2 a, float2 b, float2 c) {
+  return make_float2(fmin3(a.x, b.x, c.x), fmin3(a.y, b.y, c.y));
+}
+__device__ __forceinline__ float2 vmax3(float2 a, float2 b, float2 c) {
+  return make_float2(fmax3(a.x, b.x, c.x), fmax3(a.y, b.y, c.y));
+}
 __device__ __forceinline__ float2 vabs(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
 __device__ __forceinline__ float2 vcopysign(float2 a, float2 b) {
   return make_float2(copysignf(a.x, b.x), copysignf(a.y, b.y));
