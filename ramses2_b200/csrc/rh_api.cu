@@ -399,6 +399,7 @@ int rh_finalize(void) {
   cudaStreamSynchronize(c.stream);
   rh_batch_free();
   free_state();
+  free_host_ring();
   cudaFree(c.d_err);
   cudaFree(c.d_check);
   cudaFree(c.d_gface);
@@ -686,6 +687,11 @@ int rh_transfer_grid_host(double* uold, int ngridmax, int nvar, int twotondim) {
     return RH_EINVAL;
   }
   const long long n = c.ngridmax;
+  if (pageable(uold)) {
+    RH_CUDA(cudaStreamSynchronize(c.stream));
+    return octs_to_host(uold, OctSource{c.ud[c.cur], c.precision == RH_PREC_FP64 ? nullptr : c.uf[c.cur]}, n,
+                        c.device);
+  }
   if (c.precision == RH_PREC_FP64) {
     RH_CUDA(cudaMemcpyAsync(uold, c.ud[c.cur], sizeof(double) * 40 * n, cudaMemcpyDeviceToHost, c.stream));
   } else {

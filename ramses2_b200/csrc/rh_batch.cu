@@ -784,21 +784,9 @@ int rh_batch_fetch(int id, double* host_uold) {
   RH_CUDA(cudaStreamSynchronize(c.stream));
   int cur = 0;
   RH_CUDA(cudaMemcpy(&cur, b.d_cur + id, sizeof(int), cudaMemcpyDeviceToHost));
-  if (b.precision == RH_PREC_FP64) {
-    RH_CUDA(cudaMemcpy(host_uold, b.ud[cur] + hp.oct0 * 40, sizeof(double) * 40 * hp.noct,
-                       cudaMemcpyDeviceToHost));
-  } else {
-    std::vector<float> f((size_t)hp.noct * kBulkF);  // whole records; E read through the double view
-    RH_CUDA(cudaMemcpy(f.data(), b.uf[cur] + hp.oct0 * kBulkF, (size_t)kBulkBytes * hp.noct,
-                       cudaMemcpyDeviceToHost));
-    const double* e = reinterpret_cast<const double*>(f.data()) + kBulkE;
-    for (long long o = 0; o < hp.noct; ++o)
-      for (int cell = 0; cell < 8; ++cell) {
-        for (int v = 0; v < 4; ++v) host_uold[o * 40 + v * 8 + cell] = (double)f[o * kBulkF + v * 8 + cell];
-        host_uold[o * 40 + 32 + cell] = e[o * kBulkD + cell];
-      }
-  }
-  return RH_OK;
+  const bool bulk = b.precision == RH_PREC_FP32_BULK;
+  const OctSource src{b.ud[cur] + hp.oct0 * (bulk ? kBulkD : 40), bulk ? b.uf[cur] + hp.oct0 * kBulkF : nullptr};
+  return octs_to_host(host_uold, src, hp.noct, c.device);
 }
 
 // A problem as a one-level mesh (level 1, n/2 octs per axis, row-major octs)

@@ -203,6 +203,18 @@ __global__ void reduce_partials_kernel(const double* __restrict__ partial, long 
                                        double* __restrict__ out);
 #endif
 
+// rh_hostcopy.cu: a run of octs (FP64: uf null; FP32-bulk: ud the records' E
+// view, rh_bulk.h) to pageable host memory in the reference's FP64 layout.
+// The source is complete (its stream synchronised) before the call, the
+// destination after it.
+struct OctSource {
+  const double* ud;
+  const float* uf;
+};
+int octs_to_host(double* dst, const OctSource& s, long long noct, int device);
+bool pageable(const void* p);  // host memory CUDA has not pinned
+void free_host_ring();
+
 // restart / snapshot file images (rh_io.cu)
 struct ImageSrc {
   const double* ud = nullptr;  // FP64: [oct][5][8]; FP32-bulk: the records' E view (rh_bulk.h)
