@@ -288,16 +288,11 @@ __device__ __forceinline__ void cfl_block_reduce(const CflAcc& a, const CflConst
   }
 }
 
-// Column geometry shared by both kernels: the thread's ring column and, for
-// some threads, one outer-ring column (only converted, never traced).  Outer
-// tasks are spread over all warps so no warp carries them all.
+// Column geometry shared by both kernels: the thread's ring column.
 template <class G> struct Columns {
   int rx, ry, lc, slot;
   CellMap mx, my;
-  bool interior, in_domain_xy, in_dom_xy, has_outer;
-  int orx, ory, olc, oslot;
-  CellMap omx, omy;
-  static constexpr int kStride = G::NT / G::NOC > 0 ? G::NT / G::NOC : 1;
+  bool interior, in_domain_xy, in_dom_xy;
   __device__ __forceinline__ void init(int t, int ox0, int oy0, const LevelArgs& A) {
     rx = t % G::RW - 1;
     ry = t / G::RW - 1;
@@ -309,22 +304,47 @@ template <class G> struct Columns {
     interior = rx >= 0 && rx < G::CX && ry >= 0 && ry < G::CY;
     in_domain_xy = gx < A.ncx && gy < A.ncy;
     in_dom_xy = gx >= 0 && gy >= 0 && in_domain_xy;
-    int o = (t % kStride == 0) ? t / kStride : -1;
-    if (o >= G::NOC) o = -1;
-    has_outer = o >= 0;
-    orx = 0;
-    ory = 0;
-    if (o >= 0) {
-      if (o < G::LW) { orx = o - 2; ory = -2; }
-      else if (o < 2 * G::LW) { orx = o - G::LW - 2; ory = G::CY + 1; }
-      else if (o < 2 * G::LW + G::RH) { orx = -2; ory = o - 2 * G::LW - 1; }
-      else { orx = G::CX + 1; ory = o - 2 * G::LW - G::RH - 1; }
-    }
-    olc = (orx + 2) + (ory + 2) * G::LW;
-    omx = map_coord(2 * ox0 + orx, A.ncx, A.periodic[0], A.btype[0], A.btype[1]);
-    omy = map_coord(2 * oy0 + ory, A.ncy, A.periodic[1], A.btype[2], A.btype[3]);
-    oslot = ((orx >> 1) + 1) + G::OW * ((ory >> 1) + 1);
   }
+};
+
+// The tile's outer-ring columns (only converted, never traced), packed into as
+// few warps as hold them: spread thinly over all warps, every warp issued the
+// conversion for a few lanes.  Rings of 32 columns: the first and the last
+// warp, which hold the ring rows below and above the tile and solve no face
+// in the time this takes, two passes each.  A thread keeps its columns as
+// packed codes (load-region index, staged oct column, cell parity, velocity
+// flips).
+template <class G> struct OuterColumns {
+  static constexpr bool kRowWarps = G::RW == 32;
+  static constexpr int kFull = (G::NOC + 31) / 32 * 32;
+  static constexpr int kCount = kRowWarps ? 64 : (kFull < G::NT ? kFull : G::NT);
+  static constexpr int kPasses = (G::NOC + kCount - 1) / kCount;
+  static constexpr uint32_t kNone = 0xffffffffu;
+  uint32_t code[kPasses];
+  __device__ __forceinline__ void init(int t, int ox0, int oy0, const LevelArgs& A) {
+    const int u = kRowWarps ? (t < 32 ? t : (t >= G::NT - 32 ? t - (G::NT - 64) : G::NOC)) : (t < kCount ? t : G::NOC);
+#pragma unroll
+    for (int i = 0; i < kPasses; ++i) {
+      const int o = u + i * kCount;
+      code[i] = kNone;
+      if (o >= G::NOC) continue;
+      int rx, ry;
+      if (o < G::LW) { rx = o - 2; ry = -2; }
+      else if (o < 2 * G::LW) { rx = o - G::LW - 2; ry = G::CY + 1; }
+      else if (o < 2 * G::LW + G::RH) { rx = -2; ry = o - 2 * G::LW - 1; }
+      else { rx = G::CX + 1; ry = o - 2 * G::LW - G::RH - 1; }
+      const CellMap mx = map_coord(2 * ox0 + rx, A.ncx, A.periodic[0], A.btype[0], A.btype[1]);
+      const CellMap my = map_coord(2 * oy0 + ry, A.ncy, A.periodic[1], A.btype[2], A.btype[3]);
+      const int lc = (rx + 2) + (ry + 2) * G::LW, slot = ((rx >> 1) + 1) + G::OW * ((ry >> 1) + 1);
+      code[i] = (uint32_t)lc | (uint32_t)slot << 12 | (uint32_t)(mx.parity + 2 * my.parity) << 20 |
+                (mx.flip ? 1u << 22 : 0u) | (my.flip ? 1u << 23 : 0u);
+    }
+  }
+  static __device__ __forceinline__ int lc(uint32_t c) { return c & 0xfff; }
+  static __device__ __forceinline__ int slot(uint32_t c) { return (c >> 12) & 0xff; }
+  static __device__ __forceinline__ int parity(uint32_t c) { return (c >> 20) & 3; }
+  static __device__ __forceinline__ bool flip_x(uint32_t c) { return c >> 22 & 1; }
+  static __device__ __forceinline__ bool flip_y(uint32_t c) { return c >> 23 & 1; }
 };
 
 // Dynamic shared memory of the pencil kernels and the CTA's abort flag (set
@@ -389,25 +409,38 @@ template <typename T, class G, bool DENSE = false> struct Stager {
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
   }
+  // Oct column whose copies this thread issues (-1: none), the same number in
+  // every warp: a warp issues its lanes' copies one after the other, and the
+  // barrier of the next layer waits for the warp with the most.  (In the first
+  // NSLOT threads, full warps, 256^3 took: FP64 8x8 1.715 ms, 7x11 1.526,
+  // FP32-bulk 7x7 0.845, 15x7 0.908; spread 1.623, 1.480, 0.830, 0.858.)
+  static constexpr int kPerWarp = (G::NSLOT + G::NWARP - 1) / G::NWARP;
+  static_assert(kPerWarp <= 32, "more oct columns than threads");
+  __device__ __forceinline__ static int own_slot() {
+    const int lane = threadIdx.x & 31, s = (threadIdx.x >> 5) * kPerWarp + lane;
+    return lane < kPerWarp && s < G::NSLOT ? s : -1;
+  }
   // The table entry this thread's copy of layer row reads (-1 for threads
   // that issue none): loaded ahead of issue(row, oct), the copy does not wait
   // for the table read.
   __device__ __forceinline__ int entry(int row) const {
-    return threadIdx.x < G::NSLOT ? oct_at(row, threadIdx.x) : -1;
+    const int slot = own_slot();
+    return slot >= 0 ? oct_at(row, slot) : -1;
   }
   __device__ __forceinline__ void issue(int row) { issue(row, entry(row)); }
   __device__ __forceinline__ void issue(int row, int oct) {
-    const int t = threadIdx.x;
-    if (t < G::NSLOT) {
+    const int slot = own_slot();
+    if (slot >= 0) {
       const int st = (rb() + row) % G::NSTAGE;
       fence_proxy_async_smem();
       if (oct >= 0) {
         mbar_arrive_expect_tx(&bar[st], Store<T>::kBytes);
         if (sizeof(T) == 8) {
-          bulk_g2s(stageD + ((size_t)st * G::NSLOT + t) * Store<T>::kSlotD, src_d + (size_t)oct * 40, 320, &bar[st]);
-        } else {
-          bulk_g2s(stageF + ((size_t)st * G::NSLOT + t) * Store<T>::kSlotF, src_f + (size_t)oct * kBulkF, kBulkBytes,
+          bulk_g2s(stageD + ((size_t)st * G::NSLOT + slot) * Store<T>::kSlotD, src_d + (size_t)oct * 40, 320,
                    &bar[st]);
+        } else {
+          bulk_g2s(stageF + ((size_t)st * G::NSLOT + slot) * Store<T>::kSlotF, src_f + (size_t)oct * kBulkF,
+                   kBulkBytes, &bar[st]);
         }
       } else {
         mbar_arrive_expect_tx(&bar[st], 0);

@@ -1,0 +1,7 @@
+// Pencil-kernel instantiations: double bulk storage, 7x11-oct XY tiles (a ring
+// of 16 x 24 columns: 12 full warps, where 8x8 has 18 x 18 columns in 11, the
+// last one with four), registers sized for 1 CTA per SM.
+#include "rh_launch.h"
+namespace rh {
+static TileRegistrar<double, 7, 11, 1> reg_f64_7x11_b1;
+}
