@@ -17,7 +17,9 @@ extern "C" {
 
 /* Pencil tile of the Godunov kernel: txo x tyo octs in x,y, registers sized
  * for minb CTAs per SM, lz oct layers per pencil.  Only compiled shapes are
- * accepted (rh_list_tiles). */
+ * accepted (rh_list_tiles).  Until it is called, rh_set_mesh takes the tile
+ * and depth that suit a single complete level's size (rh_get_tile returns
+ * them): the new state and dt are the same bit for bit whatever the tile. */
 int rh_set_tile(int txo, int tyo, int minb, int lz);
 /* Tile of the coarse-fine (multi-level) kernels; before rh_set_mesh, since a
  * mesh's interpolated ghost octs follow its pencils.  Default (the fastest on

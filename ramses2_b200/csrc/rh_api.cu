@@ -474,6 +474,7 @@ int rh_set_tile(int txo, int tyo, int minb, int lz) {
   c.cfg.tyo = tyo;
   c.cfg.minb = minb;
   c.cfg.lz = lz;
+  c.cfg_set = true;
   if (c.have_mesh && c.nlevels_used == 1)
     for (int l = c.levelmin; l <= c.levelmax; ++l)
       if (c.levels[l].built) {
@@ -552,7 +553,12 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   c.grid.assign(m->grid, m->grid + nused);
   c.nlevels_used = 0;
   for (int l = c.levelmin; l <= c.levelmax; ++l) c.nlevels_used += c.noct[l] > 0;
-  const bool multi = c.nlevels_used > 1;
+  for (int l = c.levelmin; l <= c.levelmax && c.nlevels_used == 1 && !c.cfg_set; ++l) {
+    const long long nx = (long long)c.box_nx[0] << (l - 1), ny = (long long)c.box_nx[1] << (l - 1),
+                    nz = (long long)c.box_nx[2] << (l - 1);
+    if (c.noct[l] > 0 && (long long)c.noct[l] == nx * ny * nz)
+      c.cfg = choose_tile(c.precision, (int)nx, (int)ny, (int)nz, c.sm_count);
+  }
   c.levels.assign(c.levelmax + 1, LevelTables());
   // coarse-fine levels: tables first, they fix the number of ghost octs
   long long nghost = 0;

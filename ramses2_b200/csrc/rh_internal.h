@@ -68,6 +68,7 @@ struct Context {
   int precision = RH_PREC_FP64;
   int interpol_var = 0, interpol_type = 0;
   TileCfg cfg;
+  bool cfg_set = false;  // cfg chosen by rh_set_tile (else by choose_tile at rh_set_mesh)
   // mesh (host copy of the description)
   bool have_mesh = false;
   int nsubgrid = 1, levelmin = 1, levelmax = 1, ngridmax = 0;
@@ -192,6 +193,8 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
 int stage64(long long noct, double** out);
 int ensure_level_tables(int l);
 TileCfg level_cfg(int l);  // tile of level l's launches (see rh_api.cu)
+// rh_tile.cu: tile and depth of a uniform level of nxo x nyo x nzo octs
+TileCfg choose_tile(int precision, int nxo, int nyo, int nzo, int sm_count);
 // rh_hoststep.cu: releases the overlapped host-step schedule (mesh change, finalize)
 void free_host_schedule();
 #ifdef __CUDACC__

@@ -1,0 +1,65 @@
+// rh_tile.cu — the tile a uniform level takes when its user chose none.
+//
+// A CTA marches its pencil layer by layer, so a level's step takes the CTAs'
+// waves times a pencil's march: a 64^3 level cut into 8x8-octs x 32-layer
+// pencils is 16 CTAs on 148 SMs, each marching 34 layers (FP64 257 us), while
+// 128 pencils of 4 layers take 46 us; a 256^3 level fills the chip with either
+// and wants the tile with the least halo.  choose_tile() evaluates that time
+// for the compiled tiles below and the depths that cut the level's layers
+// evenly, from three rates per tile measured on a B200 (HLLC, moncen; boxes of
+// 16^3 to 256^3 cells, even and uneven; launch gap and the reduction of the
+// pencils' partials included): with one CTA on an SM or two, a pencil of L
+// layers takes start + L * layer[0 or 1] us.  On those boxes its choice is
+// within 2 % of the fastest of all tiles and depths, but for 192^3 in FP64
+// (6 %).
+#include <algorithm>
+
+#include "rh_internal.h"
+
+namespace rh {
+namespace {
+
+struct TileRate {
+  int prec, txo, tyo, minb;
+  double start, layer[2];
+};
+const TileRate kRates[] = {
+    {RH_PREC_FP64, 6, 4, 2, 15.4, {4.77, 6.03}},       {RH_PREC_FP64, 8, 4, 2, 15.7, {5.47, 6.76}},
+    {RH_PREC_FP64, 8, 8, 1, 16.5, {6.99, 6.99}},       {RH_PREC_FP64, 7, 11, 1, 16.1, {7.08, 7.08}},
+    {RH_PREC_FP64, 15, 5, 1, 16.4, {7.00, 7.00}},      {RH_PREC_FP32_BULK, 6, 4, 2, 14.9, {2.63, 3.48}},
+    {RH_PREC_FP32_BULK, 8, 4, 2, 15.0, {3.10, 3.94}},  {RH_PREC_FP32_BULK, 7, 7, 2, 15.4, {3.44, 5.15}},
+    {RH_PREC_FP32_BULK, 15, 7, 1, 16.7, {5.40, 5.40}},
+};
+constexpr double kLaunch = 2.0;  // us of start that later waves of a launch do not pay
+constexpr int kMaxDepth = 48;    // layers; longer pencils only lost to the wave count
+
+double step_us(const TileRate& r, long long pencils, int lz, int sm_count) {
+  if (pencils <= sm_count) return r.start + r.layer[0] * lz;
+  const long long slots = (long long)sm_count * r.minb, full = pencils / slots, rest = pencils % slots;
+  double t = kLaunch + full * (r.start - kLaunch + r.layer[1] * lz);
+  if (rest > 0) t += r.start - kLaunch + r.layer[rest <= sm_count ? 0 : 1] * lz;
+  return t;
+}
+
+}  // namespace
+
+TileCfg choose_tile(int precision, int nxo, int nyo, int nzo, int sm_count) {
+  TileCfg best;
+  double tbest = 1e300;
+  for (const TileRate& r : kRates) {
+    if (r.prec != precision) continue;
+    const long long cols = (long long)((nxo + r.txo - 1) / r.txo) * ((nyo + r.tyo - 1) / r.tyo);
+    for (int cuts = 1; cuts <= nzo; ++cuts) {
+      const int lz = (nzo + cuts - 1) / cuts;
+      if (lz > kMaxDepth) continue;
+      const double t = step_us(r, cols * ((nzo + lz - 1) / lz), lz, sm_count);
+      if (t < tbest) {
+        tbest = t;
+        best = TileCfg{r.txo, r.tyo, r.minb, lz};
+      }
+    }
+  }
+  return best;
+}
+
+}  // namespace rh
