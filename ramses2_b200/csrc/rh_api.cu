@@ -263,6 +263,8 @@ static void free_state() {
     c.uf[i] = nullptr;
   }
   cudaFree(c.d_cfl);
+  cudaFree(c.d_ticket);
+  c.d_ticket = nullptr;
   cudaFree(c.d_scratch);
   cudaFree(c.d_refmask);
   cudaFree(c.d_gfather);
@@ -619,6 +621,8 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
     }
   }
   RH_CUDA(cudaMalloc(&c.d_cfl, sizeof(double) * 5 * (c.levelmax + 1)));
+  RH_CUDA(cudaMalloc(&c.d_ticket, sizeof(unsigned) * (c.levelmax + 1)));
+  RH_CUDA(cudaMemsetAsync(c.d_ticket, 0, sizeof(unsigned) * (c.levelmax + 1), c.stream));
   c.cfl_gen++;
   cudaFreeHost(c.h_cfl_next);
   c.h_cfl_next = nullptr;
@@ -1158,6 +1162,11 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
   A.cfl = make_cfl(dx, gamma, smallr, smallc, courant, g);
   A.vol = dx * dx * dx;
   A.cfl_partial = fuse_cfl ? (range ? range->partial : T.d_cfl_partial) : nullptr;
+  // whole-level launches reduce their partials themselves
+  const bool reduce = fuse_cfl && !range && !(slots && slots->defer_reduce);
+  A.ticket = reduce ? c.d_ticket + l : nullptr;
+  A.cfl_out = c.d_cfl + 5 * l;
+  A.cfl_host = c.h_cfl_next + 5 * l;
   A.refmask = c.d_refmask;
   A.ghost_father = c.d_gfather;
   A.accumulate = accumulate ? 1 : 0;
@@ -1218,11 +1227,7 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
                                                          c.uf[nxt], c.ud[nxt]);
     RH_CUDA(cudaGetLastError());
   }
-  if (fuse_cfl && !range && !(slots && slots->defer_reduce)) {
-    reduce_partials_kernel<<<1, 1024, 0, st>>>(T.d_cfl_partial, T.npencil, A.cfl.cdx_smallc, c.d_cfl + 5 * l);
-    c.cfl_gen++;
-    RH_CUDA(cudaGetLastError());
-  }
+  if (reduce) c.cfl_gen++;
   return RH_OK;
 }
 
@@ -1687,11 +1692,16 @@ int rh_coarse_step(const rh_hydro_params* p, double* dt, double* cfl) {
   for (int l : lev) all_fused = all_fused && c.cfl_on_uold[l];
   if (all_fused) {
     const int l0 = lev.front(), nl = lev.back() - l0 + 1;
-    RH_CUDA(cudaEventRecord(c.ev_cfl_ready, c.stream));
-    RH_CUDA(cudaStreamWaitEvent(c.cfl_copy, c.ev_cfl_ready, 0));
-    RH_CUDA(cudaMemcpyAsync(c.h_cfl_next + 5 * l0, c.d_cfl + 5 * l0, sizeof(double) * 5 * nl,
-                            cudaMemcpyDeviceToHost, c.cfl_copy));
-    RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.cfl_copy));
+    if (nl == 1) {
+      // a single level's step left them in h_cfl_next itself
+      RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.stream));
+    } else {
+      RH_CUDA(cudaEventRecord(c.ev_cfl_ready, c.stream));
+      RH_CUDA(cudaStreamWaitEvent(c.cfl_copy, c.ev_cfl_ready, 0));
+      RH_CUDA(cudaMemcpyAsync(c.h_cfl_next + 5 * l0, c.d_cfl + 5 * l0, sizeof(double) * 5 * nl,
+                              cudaMemcpyDeviceToHost, c.cfl_copy));
+      RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.cfl_copy));
+    }
     c.cfl_next_gen = c.cfl_gen;
     c.cfl_next_l0 = l0;
     c.cfl_next_l1 = lev.back();

@@ -75,6 +75,9 @@ __device__ __forceinline__ void batch_level(const BatchProb& P, double dt, int* 
   for (int i = 0; i < 6; ++i) A.btype[i] = P.btype[i];
   A.ghost_base = 0x7fffffff;
   A.cfl_partial = nullptr;
+  A.ticket = nullptr;
+  A.cfl_out = nullptr;
+  A.cfl_host = nullptr;
   A.err = err;
   A.cfl.gamma = P.gamma;
   A.cfl.gm1 = P.gamma - 1.0;

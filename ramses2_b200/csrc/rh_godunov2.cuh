@@ -98,6 +98,7 @@ godunov_pencil2_kernel(const LevelArgs A, const StateArgs<float> S, const HydroK
   const int4 hdr = A.phdr[blockIdx.x];
   const int* tab = A.ptab + A.poff[blockIdx.x];
 #include "rh_pencil_f32.inc"
+  if (A.ticket) reduce_last<G::NT>(A, red);
 }
 
 }  // namespace rh

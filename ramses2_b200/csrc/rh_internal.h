@@ -94,6 +94,7 @@ struct Context {
   unsigned* d_check = nullptr;    // [levelmax+1][3] state check results (rh_check.cu)
   int check_cap = 0;
   double* d_cfl = nullptr;        // [levelmax+1][5] reduced CFL values
+  unsigned* d_ticket = nullptr;   // [levelmax+1] CTAs done of a level's launch (zero between launches)
   double* d_scratch = nullptr;    // standalone cmpdt partials
   double* h_cfl = nullptr;        // pinned: courant_fine values read back, 5 per level
   size_t h_cfl_elems = 0;
