@@ -289,8 +289,10 @@ static void free_state() {
 static int build_level_tables(int l, const TileCfg& cfg) {
   Context& c = ctx();
   LevelTables& T = c.levels[l];
+  const bool box = T.complete_box;
   free_tables(T);
   T.cfg = cfg;
+  T.complete_box = box;
   int rc = build_complete_tables_device(l, cfg, T);
   if (rc) return rc;
   T.npencil = (int)T.phdr.size();
@@ -507,8 +509,9 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   int rc = check_ready(false);
   if (rc) return rc;
   Context& c = ctx();
-  // coarse-fine tile unless chosen: the fastest on the AMR Sedov of levels 7-10 per precision
-  if (!c.amr_cfg_set) c.amr_cfg = c.precision == RH_PREC_FP32_BULK ? TileCfg{7, 7, 2, 32} : TileCfg{8, 4, 2, 32};
+  // coarse-fine tile unless chosen: the fastest on AMR Sedovs per precision
+  // (FP64 on levels 6-9: 7x11 0.52 ms a coarse step, 8x4 0.58, 15x5 0.60)
+  if (!c.amr_cfg_set) c.amr_cfg = c.precision == RH_PREC_FP32_BULK ? TileCfg{7, 7, 2, 32} : TileCfg{7, 11, 1, 32};
   if (!m || !uold || !m->grid || !m->head || !m->noct) {
     set_error("rh_set_mesh: null pointer");
     return RH_EINVAL;
@@ -576,7 +579,8 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
     if (c.noct[l] == 0) continue;
     const long long box = ((long long)c.box_nx[0] << (l - 1)) * ((long long)c.box_nx[1] << (l - 1)) *
                           ((long long)c.box_nx[2] << (l - 1));
-    if ((long long)c.noct[l] == box) continue;
+    c.levels[l].complete_box = (long long)c.noct[l] == box;
+    if (c.levels[l].complete_box) continue;
     const long long gbase = (long long)c.ngridmax + nghost;
     // A small level gets shorter pencils so that it still fills a wave of
     // CTAs (its pencils are few; each one marches lz layers one after the
@@ -927,14 +931,25 @@ __global__ void coarse_gather_kernel(const double* __restrict__ gface, int nghos
 // Tile of level l's launches: the uniform tile on a single-level mesh, the
 // coarse-fine tile (kernels that handle refined cells and interpolated ghosts)
 // on every level of a multi-level mesh.  A partial level takes the tile's
-// layers cut down by rh_set_mesh until it fills a wave of CTAs; a
-// complete level takes them all (on the AMR Sedov of levels 7-10, whose
-// level 7 is complete, 32 layers there instead of 8 made the coarse step
-// 4 % (FP32-bulk) and 1.4 % (FP64) faster, 64 layers 30 % / 20 % slower).
+// layers cut down by rh_set_mesh until it fills a wave of CTAs.  A complete
+// level is the coarsest and runs beside the others (rh_coarse_step), so its
+// pencils may be as deep as the whole mesh's work is long: on levels 7-10 32
+// layers made the coarse step 4 % (FP32-bulk) and 1.4 % (FP64) faster than 8;
+// on levels 6-8, whose work is 7 layers of every CTA slot, its 32 layers were
+// the step (FP64 327 us a coarse step, 188 with 4 layers; through the leaf
+// calls 588 and 330).  Unless the tile was chosen by rh_set_amr_tile, the depth is
+// halved, down to 4, while a pencil's march is longer than that work.
 TileCfg level_cfg(int l) {
   Context& c = ctx();
-  (void)l;
-  return c.nlevels_used > 1 ? c.amr_cfg : c.cfg;
+  if (c.nlevels_used <= 1) return c.cfg;
+  TileCfg t = c.amr_cfg;
+  if (!c.amr_cfg_set && c.levels[l].complete_box) {
+    long long octs = 0;
+    for (int k = c.levelmin; k <= c.levelmax; ++k) octs += c.noct[k];
+    const long long layer = (long long)t.txo * t.tyo * c.sm_count * t.minb;  // octs of one layer of every CTA slot
+    while (t.lz > 4 && (t.lz + 2) * layer > octs) t.lz /= 2;
+  }
+  return t;
 }
 
 // The same for FP32-bulk records: the four float variables and the FP64

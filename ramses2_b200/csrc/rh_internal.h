@@ -30,7 +30,8 @@ struct TileCfg {
 // Pencil tables of one level (device + host copies).
 struct LevelTables {
   bool built = false;
-  bool complete = false;  // level covers its whole box (uniform level)
+  bool complete = false;  // tables of a level that covers its whole box (uniform level)
+  bool complete_box = false;  // the level covers its whole box
   // coarse-fine levels: interpolated ghost octs [gbase, gbase + nghost) of the
   // state arrays, prolonged from level l-1 before each Godunov step
   long long gbase = 0;
