@@ -49,6 +49,8 @@ struct Batch {
   bool inited = false;
   int precision = RH_PREC_FP64, slope = 2, riemann = 3;
   TileCfg cfg{8, 4, 2, 16};
+  bool cfg_set = false;          // cfg chosen by rh_batch_set_tile: its depth is taken as it is
+  int lz = 16;                   // layers per pencil of the current work list
   long long pool_octs = 0;
   int parity = 0;
   double* ud[2] = {nullptr, nullptr};
@@ -318,7 +320,7 @@ BatchProb make_prob(const rh_batch_problem& p, long long oct0) {
   P.ndim = p.ndim;
   P.tx = (p.n[0] / 2 + b.cfg.txo - 1) / b.cfg.txo;
   P.ty = (p.n[1] / 2 + b.cfg.tyo - 1) / b.cfg.tyo;
-  P.tz = (p.n[2] / 2 + b.cfg.lz - 1) / b.cfg.lz;
+  P.tz = (p.n[2] / 2 + b.lz - 1) / b.lz;
   // 2D problems on the plane path: one work item per kPlaneGroup tile bodies
   // along y (FP32-bulk tile bodies take two tile rows, one per lane)
   if (b.plane2d && p.ndim == 2 && p.n[2] == 2 && P.periodic[2]) {
@@ -356,8 +358,22 @@ int rebuild() {
   std::sort(ids.begin(), ids.end(), [&](int x, int y) { return b.probs[x].noct > b.probs[y].noct; });
   std::vector<long long> woff(ids.size() + 1, 0);
   std::vector<BatchProb> probs(b.cap);
-  for (int i = 0; i < b.cap; ++i)
-    if (b.probs[i].used) probs[i] = make_prob(b.probs[i].p, b.probs[i].oct0);
+  // Pencil depth: the tile's, halved (down to 2) while the batch does not make
+  // a work item for every CTA slot: a few small problems are a few deep pencils,
+  // each marched by one CTA while the others idle (12 FP64 problems of 16^3 to
+  // 64^3: 0.247 -> 0.187 ms a step).  States, times and dt do
+  // not depend on it (a cell's update does not depend on where pencils end, the
+  // dt is a minimum); the conserved totals are summed in another order.
+  const long long slots = (long long)std::max(1, b.cfg.minb) * c.sm_count;
+  b.lz = b.cfg.lz;
+  for (;; b.lz /= 2) {
+    long long work = 0;
+    for (int i : ids) {
+      probs[i] = make_prob(b.probs[i].p, b.probs[i].oct0);
+      work += (long long)probs[i].tx * probs[i].ty * probs[i].tz;
+    }
+    if (b.cfg_set || b.lz <= 2 || work >= slots) break;
+  }
   for (size_t s = 0; s < ids.size(); ++s) {
     const BatchProb& P = probs[ids[s]];
     woff[s + 1] = woff[s] + (long long)P.tx * P.ty * P.tz;
@@ -409,7 +425,7 @@ int rebuild() {
     RH_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     for (int h = 0; h < 2; ++h) {
       const int par = (b.parity + h) & 1;
-      BatchArgs A{b.d_prob, b.d_order, b.d_woff, b.nslot, b.nwork, b.cfg.txo, b.cfg.tyo, b.cfg.lz, b.d_counter,
+      BatchArgs A{b.d_prob, b.d_order, b.d_woff, b.nslot, b.nwork, b.cfg.txo, b.cfg.tyo, b.lz, b.d_counter,
                   b.d_done, b.d_dt, b.d_partial, {b.ud[0], b.ud[1]}, {b.uf[0], b.uf[1]}, c.d_err,
                   b.plane2d};
       cudaError_t e = reg->fn(A, par, b.nblocks, c.stream);
@@ -662,6 +678,7 @@ int rh_batch_set_tile(int txo, int tyo, int minb, int lz) {
     return RH_EINVAL;
   }
   b.cfg = TileCfg{txo, tyo, minb, lz};
+  b.cfg_set = true;
   b.dirty = true;
   return RH_OK;
 }
@@ -697,7 +714,7 @@ int rh_batch_step(int nsteps) {
       RH_CUDA(cudaGraphLaunch(b.graph, c.stream));
       done_steps += 2;
     } else {
-      BatchArgs A{b.d_prob, b.d_order, b.d_woff, b.nslot, b.nwork, b.cfg.txo, b.cfg.tyo, b.cfg.lz, b.d_counter,
+      BatchArgs A{b.d_prob, b.d_order, b.d_woff, b.nslot, b.nwork, b.cfg.txo, b.cfg.tyo, b.lz, b.d_counter,
                   b.d_done, b.d_dt, b.d_partial, {b.ud[0], b.ud[1]}, {b.uf[0], b.uf[1]}, c.d_err,
                   b.plane2d};
       RH_CUDA(reg->fn(A, b.parity, b.nblocks, c.stream));
