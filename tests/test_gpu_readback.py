@@ -34,7 +34,7 @@ def as_stored(u, prec):
 def test_batch_fetch_returns_the_state_at_every_copy_size(prec, pinned):
     import torch
 
-    sizes = (1, 4095, 4096, 13056, 13057, 2 * 13056, 9 * 13056 + 5)
+    sizes = (1, 1631, 1632, 1633, 16 * 1632, 16 * 1632 + 17, 17 * 13056 + 5)
     b = Batch(prec, pool_octs=sum(sizes))
     try:
         want = {}
