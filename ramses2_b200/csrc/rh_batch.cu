@@ -347,6 +347,25 @@ void check_step(int parity) {
       b.precision == RH_PREC_FP32_BULK ? 1 : 0, b.d_bad);
 }
 
+// Tile of a batch whose user chose none: 8x4, the fastest on uneven 3D
+// ensembles in both precisions, whose boxes of 8 to 64 octs it divides (96
+// problems of 16^3 to 128^3, FP32-bulk: 3.00 ms a step, 7x7 3.22, 8x8 3.30; FP64:
+// 5.08, 8x8 5.49).  The FP32-bulk plane body of 2D problems is faster on 7x7
+// (twelve of 256^2 to 1024^2: 0.483 against 0.496 ms), which mostly 2D batches
+// take: from twice the 3D cells on, its 2.6 % outweigh the 3D problems' 7 %.
+TileCfg default_tile(const std::vector<int>& ids) {
+  Batch& b = B();
+  if (b.precision == RH_PREC_FP32_BULK) {
+    long long plane = 0, cube = 0;
+    for (int i : ids) {
+      const rh_batch_problem& p = b.probs[i].p;
+      (p.ndim == 2 ? plane : cube) += b.probs[i].noct * (p.ndim == 2 ? 4 : 8);
+    }
+    if (plane > 2 * cube) return TileCfg{7, 7, 2, 32};
+  }
+  return TileCfg{8, 4, 2, 32};
+}
+
 // Rebuild the work list (largest problems first) and the step graph.
 int rebuild() {
   Batch& b = B();
@@ -364,6 +383,7 @@ int rebuild() {
   // 64^3: 0.247 -> 0.187 ms a step).  States, times and dt do
   // not depend on it (a cell's update does not depend on where pencils end, the
   // dt is a minimum); the conserved totals are summed in another order.
+  if (!b.cfg_set) b.cfg = default_tile(ids);
   const long long slots = (long long)std::max(1, b.cfg.minb) * c.sm_count;
   b.lz = b.cfg.lz;
   for (;; b.lz /= 2) {
@@ -481,9 +501,7 @@ int rh_batch_init(int precision, int slope, int riemann, long long pool_octs) {
   b.slope = slope;
   b.riemann = riemann;
   b.pool_octs = pool_octs;
-  // default tile per precision: the fastest of the autotuner's sweep on the
-  // uneven 3D ensemble and on mixed 2D/3D serving
-  b.cfg = precision == RH_PREC_FP32_BULK ? TileCfg{7, 7, 2, 32} : TileCfg{8, 4, 2, 32};
+  b.cfg = default_tile({});
   b.cap = 4096;
   for (int i = 0; i < 2; ++i) {
     if (precision == RH_PREC_FP64) {
