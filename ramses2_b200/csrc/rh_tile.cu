@@ -3,15 +3,13 @@
 // A CTA marches its pencil layer by layer, so a level's step takes the CTAs'
 // waves times a pencil's march: a 64^3 level cut into 8x8-octs x 32-layer
 // pencils is 16 CTAs on 148 SMs, each marching 34 layers (FP64 257 us), while
-// 128 pencils of 4 layers take 46 us; a 256^3 level fills the chip with either
+// 256 pencils of 8x4 octs x 4 layers take 41 us; a 256^3 level fills the chip with either
 // and wants the tile with the least halo.  choose_tile() evaluates that time
 // for the compiled tiles below and the depths that cut the level's layers
 // evenly, from three rates per tile measured on a B200 (HLLC, moncen; boxes of
-// 16^3 to 256^3 cells, even and uneven; launch gap and the reduction of the
-// pencils' partials included): with one CTA on an SM or two, a pencil of L
-// layers takes start + L * layer[0 or 1] us.  On those boxes its choice is
-// within 2 % of the fastest of all tiles and depths, but for 192^3 in FP64
-// (6 %).
+// 16^3 to 256^3 cells, even and uneven; launch gap included): with one CTA on
+// an SM or two, a pencil of L layers takes start + L * layer[0 or 1] us.  On
+// those boxes its choice is within 1 % of the fastest of all tiles and depths.
 #include <algorithm>
 
 #include "rh_internal.h"
@@ -24,11 +22,11 @@ struct TileRate {
   double start, layer[2];
 };
 const TileRate kRates[] = {
-    {RH_PREC_FP64, 6, 4, 2, 15.4, {4.77, 6.03}},       {RH_PREC_FP64, 8, 4, 2, 15.7, {5.47, 6.76}},
-    {RH_PREC_FP64, 8, 8, 1, 16.5, {6.99, 6.99}},       {RH_PREC_FP64, 7, 11, 1, 16.1, {7.08, 7.08}},
-    {RH_PREC_FP64, 15, 5, 1, 16.4, {7.00, 7.00}},      {RH_PREC_FP32_BULK, 6, 4, 2, 14.9, {2.63, 3.48}},
-    {RH_PREC_FP32_BULK, 8, 4, 2, 15.0, {3.10, 3.94}},  {RH_PREC_FP32_BULK, 7, 7, 2, 15.4, {3.44, 5.15}},
-    {RH_PREC_FP32_BULK, 15, 7, 1, 16.7, {5.40, 5.40}},
+    {RH_PREC_FP64, 6, 4, 2, 12.7, {4.76, 6.01}},       {RH_PREC_FP64, 8, 4, 2, 12.6, {5.51, 6.82}},
+    {RH_PREC_FP64, 8, 8, 1, 13.8, {7.00, 7.00}},       {RH_PREC_FP64, 7, 11, 1, 12.8, {6.88, 6.88}},
+    {RH_PREC_FP64, 15, 5, 1, 13.1, {6.71, 6.71}},      {RH_PREC_FP32_BULK, 6, 4, 2, 12.5, {2.56, 3.44}},
+    {RH_PREC_FP32_BULK, 8, 4, 2, 12.2, {3.08, 3.89}},  {RH_PREC_FP32_BULK, 7, 7, 2, 12.6, {3.20, 4.99}},
+    {RH_PREC_FP32_BULK, 8, 8, 1, 13.6, {3.88, 3.88}},  {RH_PREC_FP32_BULK, 15, 7, 1, 14.2, {5.45, 5.45}},
 };
 constexpr double kLaunch = 2.0;  // us of start that later waves of a launch do not pay
 constexpr int kMaxDepth = 48;    // layers; longer pencils only lost to the wave count
