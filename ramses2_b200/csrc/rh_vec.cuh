@@ -54,6 +54,10 @@ __device__ __forceinline__ double vsqrt(double x) {
   return fma(fma(e, 0.375, 0.5), s * e, s);
 }
 
+// a - b rounded once, never merged into a multiply-add with the products that
+// formed a or b
+__device__ __forceinline__ double vsub_nc(double a, double b) { return __dsub_rn(a, b); }
+
 // ---------------------------------------------------------------- float2 ---
 struct M2 {
   bool x, y;
