@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -419,6 +421,7 @@ int rh_finalize(void) {
   cudaEventDestroy(c.ev_cfl_ready);
   cudaStreamDestroy(c.cfl_copy);
   cudaFreeHost(c.h_cfl_next);
+  cudaFreeHost(c.h_cfl_seq);
   for (auto s : c.lev_stream) cudaStreamDestroy(s);
   cudaStreamDestroy(c.stream);
   c = Context();
@@ -631,6 +634,11 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   cudaFreeHost(c.h_cfl_next);
   c.h_cfl_next = nullptr;
   RH_CUDA(cudaMallocHost(&c.h_cfl_next, sizeof(double) * 5 * (c.levelmax + 1)));
+  cudaFreeHost(c.h_cfl_seq);
+  c.h_cfl_seq = nullptr;
+  RH_CUDA(cudaMallocHost(&c.h_cfl_seq, sizeof(unsigned long long) * (c.levelmax + 1)));
+  std::fill(c.h_cfl_seq, c.h_cfl_seq + c.levelmax + 1, 0ull);
+  c.cfl_seq_of.assign(c.levelmax + 1, 0);
   {
     std::vector<uint8_t> ref((size_t)n, 0);
     for (long long i = 0; i < nused; ++i) {
@@ -805,6 +813,25 @@ int rh_set_uold(int head_idx, int num_octs) {
 
 }  // extern "C"
 
+// Waits for the values that level l's last launch leaves in h_cfl_next (call
+// with cfl_seq_of[l] != 0).  The host sees them as they are written, without
+// the end of the kernel, an event and a copy in between (steps of 16^3 FP32-bulk
+// 22.5 -> 20.5 us, of 64^3 FP64 48.3 -> 45.8); after 5 ms it waits for the stream, which also reports a failed kernel.
+static int wait_cfl(int l) {
+  Context& c = ctx();
+  const volatile unsigned long long* seq = c.h_cfl_seq + l;
+  const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(5);
+  for (int i = 0; *seq != c.cfl_seq_of[l]; ++i)
+    if ((i & 255) == 255 && std::chrono::steady_clock::now() > until) {
+      RH_CUDA(cudaStreamSynchronize(c.stream));
+      if (*seq == c.cfl_seq_of[l]) break;
+      set_error("courant_fine values of level %d did not arrive", l);
+      return RH_ECUDA;
+    }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return RH_OK;
+}
+
 // courant_fine of one level range, queued on the library stream: the five
 // reduced values land in host_out (pinned) once the stream reaches them.
 // *queued is false when there is nothing to wait for (an empty range).
@@ -853,6 +880,7 @@ static int cmpdt_enqueue(int head_idx, int num_octs, double dx, double gamma, do
     RH_CUDA(cudaGetLastError());
     RH_CUDA(cudaMemcpyAsync(host_out, d_out, sizeof(double) * 5, cudaMemcpyDeviceToHost, c.stream));
     if (l >= 0) c.cfl_on_uold[l] = 0;
+    if (l >= 0) c.cfl_seq_of[l] = 0;
   }
   if (lkey) std::copy(key, key + 8, lkey);
   *queued = true;
@@ -1182,6 +1210,8 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
   A.ticket = reduce ? c.d_ticket + l : nullptr;
   A.cfl_out = c.d_cfl + 5 * l;
   A.cfl_host = c.h_cfl_next + 5 * l;
+  A.seq_host = c.h_cfl_seq + l;
+  A.seq = c.cfl_seq + 1;
   A.refmask = c.d_refmask;
   A.ghost_father = c.d_gfather;
   A.accumulate = accumulate ? 1 : 0;
@@ -1242,7 +1272,12 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
                                                          c.uf[nxt], c.ud[nxt]);
     RH_CUDA(cudaGetLastError());
   }
-  if (reduce) c.cfl_gen++;
+  if (reduce) {
+    c.cfl_gen++;
+    c.cfl_seq_of[l] = ++c.cfl_seq;
+  } else if (fuse_cfl) {
+    c.cfl_seq_of[l] = 0;
+  }
   return RH_OK;
 }
 
@@ -1450,7 +1485,10 @@ int rh_coarse_step(const rh_hydro_params* p, double* dt, double* cfl) {
       all_cached = all_cached && c.cfl_on_uold[l] && std::equal(key, key + 8, &c.cfl_keys[8 * l]);
     }
     const int l0 = lev.empty() ? 0 : lev.front(), nl = lev.empty() ? 0 : lev.back() - l0 + 1;
-    if (all_cached && c.cfl_next_gen == c.cfl_gen && c.cfl_next_l0 == l0 && c.cfl_next_l1 == lev.back()) {
+    if (all_cached && lev.size() == 1 && c.cfl_seq_of[l0]) {
+      if ((rc = wait_cfl(l0))) return rc;
+      std::copy(c.h_cfl_next + 5 * l0, c.h_cfl_next + 5 * l0 + 5, h + 5 * l0);
+    } else if (all_cached && c.cfl_next_gen == c.cfl_gen && c.cfl_next_l0 == l0 && c.cfl_next_l1 == lev.back()) {
       // copied by the previous call as soon as they were final: no wait
       // for the rest of that step (its restrictions)
       RH_CUDA(cudaEventSynchronize(c.ev_cfl_copied));
@@ -1705,18 +1743,13 @@ int rh_coarse_step(const rh_hydro_params* p, double* dt, double* cfl) {
   // on their way to the host before the next call asks for them
   bool all_fused = !lev.empty();
   for (int l : lev) all_fused = all_fused && c.cfl_on_uold[l];
-  if (all_fused) {
+  if (all_fused && lev.size() > 1) {  // (a single level's step leaves them there itself)
     const int l0 = lev.front(), nl = lev.back() - l0 + 1;
-    if (nl == 1) {
-      // a single level's step left them in h_cfl_next itself
-      RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.stream));
-    } else {
-      RH_CUDA(cudaEventRecord(c.ev_cfl_ready, c.stream));
-      RH_CUDA(cudaStreamWaitEvent(c.cfl_copy, c.ev_cfl_ready, 0));
-      RH_CUDA(cudaMemcpyAsync(c.h_cfl_next + 5 * l0, c.d_cfl + 5 * l0, sizeof(double) * 5 * nl,
-                              cudaMemcpyDeviceToHost, c.cfl_copy));
-      RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.cfl_copy));
-    }
+    RH_CUDA(cudaEventRecord(c.ev_cfl_ready, c.stream));
+    RH_CUDA(cudaStreamWaitEvent(c.cfl_copy, c.ev_cfl_ready, 0));
+    RH_CUDA(cudaMemcpyAsync(c.h_cfl_next + 5 * l0, c.d_cfl + 5 * l0, sizeof(double) * 5 * nl,
+                            cudaMemcpyDeviceToHost, c.cfl_copy));
+    RH_CUDA(cudaEventRecord(c.ev_cfl_copied, c.cfl_copy));
     c.cfl_next_gen = c.cfl_gen;
     c.cfl_next_l0 = l0;
     c.cfl_next_l1 = lev.back();

@@ -78,6 +78,8 @@ __device__ __forceinline__ void batch_level(const BatchProb& P, double dt, int* 
   A.ticket = nullptr;
   A.cfl_out = nullptr;
   A.cfl_host = nullptr;
+  A.seq_host = nullptr;
+  A.seq = 0;
   A.err = err;
   A.cfl.gamma = P.gamma;
   A.cfl.gm1 = P.gamma - 1.0;

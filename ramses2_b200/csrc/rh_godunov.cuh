@@ -128,7 +128,9 @@ struct LevelArgs {
   // with a ticket the launch's last CTA reduces the partials (reduce_last)
   unsigned* ticket;       // CTAs done, zero between launches; null: no reduction
   double* cfl_out;        // the level's five reduced values
-  double* cfl_host;       // the same in pinned host memory, or null
+  double* cfl_host;       // the same in pinned host memory, then the number of
+  unsigned long long* seq_host;  // the launch (seq), for the host to see them by
+  unsigned long long seq;
   CflConst cfl;
   double vol;
   double gm1_d, smalle_d;  // FP64 pressure recovery constants
@@ -338,9 +340,11 @@ template <int NT> __device__ __forceinline__ void reduce_last(const LevelArgs& A
     const double out[5] = {v[0], v[1], v[2], 0.0, d};
     for (int n = 0; n < 5; ++n) {
       A.cfl_out[n] = out[n];
-      if (A.cfl_host) A.cfl_host[n] = out[n];
+      A.cfl_host[n] = out[n];
     }
     *A.ticket = 0;
+    __threadfence_system();
+    *(volatile unsigned long long*)A.seq_host = A.seq;
   }
 }
 

@@ -105,6 +105,12 @@ struct Context {
   // from there while cfl_next_gen still equals cfl_gen.
   unsigned long long cfl_gen = 0, cfl_next_gen = ~0ull;
   double* h_cfl_next = nullptr;   // pinned, 5 per level
+  // A launch that reduces its own partials (LevelArgs::ticket) stores the
+  // level's values there and then its number in h_cfl_seq; cfl_seq_of is the
+  // number whose values are the level's current ones (0: they came otherwise).
+  unsigned long long* h_cfl_seq = nullptr;  // pinned, one per level
+  unsigned long long cfl_seq = 0;
+  std::vector<unsigned long long> cfl_seq_of;
   int cfl_next_l0 = -1, cfl_next_l1 = -1;
   cudaStream_t cfl_copy = nullptr;
   cudaEvent_t ev_cfl_copied = nullptr, ev_cfl_ready = nullptr;
