@@ -14,8 +14,8 @@
 // queues, made the copies queue behind kernels (26.6 ms per 256^3 step
 // against 18.1).
 // The pencil kernel is the one rh_coarse_step runs (the level's tile shape),
-// launched group by group over the schedule's own pencil tables, 2 (FP32-bulk)
-// or 8 (FP64) layers deep.  A cell's update does not depend on where pencils
+// launched group by group over the schedule's own pencil tables, 2 layers
+// deep.  A cell's update does not depend on where pencils
 // start and end, so the new state is bitwise that of rh_set_grid_device +
 // rh_coarse_step + rh_transfer_grid_host, and so is the next dt (a minimum);
 // the conserved totals of the fused CFL epilogue are summed over other
@@ -44,7 +44,7 @@ struct HostStepSched {
   // what the schedule was built for: level, kernel tile shape, precision
   int level = -1, txo = 0, tyo = 0, minb = 0, precision = -1;
   long long noct = 0;
-  // the schedule's own pencil tables: the level's tile shape, sched_lz() layers deep
+  // the schedule's own pencil tables: the level's tile shape, kSchedLz layers deep
   LevelTables T;
   int npencil = 0;
   // chunks: [k*C, min((k+1)*C, noct)) octs; uploaded in the order up_order
@@ -66,13 +66,10 @@ namespace {
 
 // Pencils this deep: a pencil needs its neighbourhood and a chunk waits for
 // the pencils that write it, so shallow pencils start earlier and release
-// chunks sooner; the pencils' extra halo work is hidden behind the copies.
-// FP32-bulk takes 2 layers, FP64 8: on a 256^3 step 2 layers brought the
-// FP32-bulk step from 18.7 to 18.2 ms (the first chunks go back sooner, and
-// the extra halo work of its fast kernel stays hidden behind the copies) and
-// the FP64 one from 16.3 to 18.2 ms (its kernel, twice as slow, no longer
-// keeps pace).
-int sched_lz(int precision) { return precision == RH_PREC_FP32_BULK ? 2 : 8; }
+// chunks sooner; their extra halo work is hidden behind the copies.  Steps with
+// 2 and with 8 layers: 256^3 18.1 / 18.4 ms FP32-bulk, 17.8 / 18.3 FP64; 64^3
+// 0.46 / 0.47 and 0.46 / 0.49; 32^3 0.120 / 0.139 and 0.116 / 0.149.
+constexpr int kSchedLz = 2;
 // 128 chunks of 16,384 octs (5.2 MB of FP64 state per copy) for a 256^3
 // level: on one box 18.8-18.9 ms per FP32-bulk step, against 18.3-19.6 with
 // 256 chunks and 20-21 with 64 (fewer chunks leave a longer tail of downloads
@@ -107,7 +104,7 @@ int build_sched(int l, HostStepSched& S) {
   const long long o0 = c.head[l] - 1;  // 0 for the single level of a mesh
   const TileCfg& main = c.cfg;
   TileCfg cfg = main;
-  cfg.lz = sched_lz(c.precision);
+  cfg.lz = kSchedLz;
   S.level = l;
   S.txo = main.txo;
   S.tyo = main.tyo;
