@@ -349,10 +349,11 @@ void check_step(int parity) {
 
 // Tile of a batch whose user chose none: 8x4, the fastest on uneven 3D
 // ensembles in both precisions, whose boxes of 8 to 64 octs it divides (96
-// problems of 16^3 to 128^3, FP32-bulk: 3.00 ms a step, 7x7 3.22, 8x8 3.30; FP64:
-// 5.08, 8x8 5.49).  The FP32-bulk plane body of 2D problems is faster on 7x7
+// problems of 16^3 to 128^3, FP32-bulk: 2.85 ms a step, 7x7 3.22; FP64: 5.08, 8x8
+// 5.49).  The FP32-bulk plane body of 2D problems is faster on 7x7
 // (twelve of 256^2 to 1024^2: 0.483 against 0.496 ms), which mostly 2D batches
-// take: from twice the 3D cells on, its 2.6 % outweigh the 3D problems' 7 %.
+// take: from four times the 3D cells on, its 2.6 % outweigh the 3D problems'
+// 11 %.
 TileCfg default_tile(const std::vector<int>& ids) {
   Batch& b = B();
   if (b.precision == RH_PREC_FP32_BULK) {
@@ -361,7 +362,7 @@ TileCfg default_tile(const std::vector<int>& ids) {
       const rh_batch_problem& p = b.probs[i].p;
       (p.ndim == 2 ? plane : cube) += b.probs[i].noct * (p.ndim == 2 ? 4 : 8);
     }
-    if (plane > 2 * cube) return TileCfg{7, 7, 2, 32};
+    if (plane > 4 * cube) return TileCfg{7, 7, 2, 32};
   }
   return TileCfg{8, 4, 2, 32};
 }

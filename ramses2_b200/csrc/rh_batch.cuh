@@ -123,6 +123,9 @@ template <class V> __device__ __forceinline__ void batch_hydro(const BatchProb& 
   H.grav[0] = H.grav[1] = H.grav[2] = b(0.0);
 }
 
+template <typename T, typename V, int TXO, int TYO>
+using BatchGeo = std::conditional_t<sizeof(T) == 8, Geo<T, V, TXO, TYO>, BatchGeo2<TXO, TYO>>;
+
 // Constants of the CTA's current work item, in shared memory: the pencil
 // body reads them where it uses them instead of holding them in registers.
 __shared__ LevelArgs rh_bA;
@@ -165,7 +168,7 @@ __device__ __noinline__ void batch_plane(int g, CflAcc* acc) {
 
 template <typename T, typename V, int TXO, int TYO, int MINB, int SLOPE, int RIEMANN>
 __global__ void __launch_bounds__(Geo<T, V, TXO, TYO>::NT, MINB) batch_step_kernel(const BatchArgs B, int parity) {
-  using G = Geo<T, V, TXO, TYO>;
+  using G = BatchGeo<T, V, TXO, TYO>;
   static_assert(G::NSLOT <= kBatchMaxSlots, "tile too wide for the dense offset table");
   __shared__ long long s_w;
   __shared__ int s_skip, s_plane;
@@ -266,7 +269,7 @@ void register_batch_launcher(const BatchKey& k, BatchLaunchFn fn, const void* fu
 
 template <typename T, typename V, int TXO, int TYO, int MINB, int SLOPE, int RIEMANN>
 cudaError_t launch_batch(const BatchArgs& B, int parity, int nblocks, cudaStream_t st) {
-  using G = Geo<T, V, TXO, TYO>;
+  using G = BatchGeo<T, V, TXO, TYO>;
   // the dynamic shared-memory attribute is set by the runtime before any launch or capture
   batch_step_kernel<T, V, TXO, TYO, MINB, SLOPE, RIEMANN><<<nblocks, G::NT, G::kSmem, st>>>(B, parity);
   return cudaGetLastError();
@@ -275,7 +278,7 @@ cudaError_t launch_batch(const BatchArgs& B, int parity, int nblocks, cudaStream
 template <typename T, int TXO, int TYO, int MINB> struct BatchRegistrar {
   BatchRegistrar() {
     using V = typename std::conditional<sizeof(T) == 8, double, float2>::type;
-    using G = Geo<T, V, TXO, TYO>;
+    using G = BatchGeo<T, V, TXO, TYO>;
     constexpr int P = sizeof(T) == 8 ? RH_PREC_FP64 : RH_PREC_FP32_BULK;
 #define RH_BREG(S, R)                                                                              \
   register_batch_launcher({P, TXO, TYO, MINB, S, R}, &launch_batch<T, V, TXO, TYO, MINB, S, R>,  \

@@ -59,7 +59,13 @@ template <> struct Store<float> {  // FP32-bulk: one 192-byte record per oct (rh
 
 // NQ: primitive planes (or FP32-bulk oct layers) kept in shared memory: 2 for
 // slopes along the three axes, 3 for the 27-point limiter of slope_type 3.
-template <typename T, typename V, int TXO, int TYO, int NQ = 2> struct Geo {
+// KEEP (FP32-bulk): the conserved values of the cells of two layers stay in
+// shared memory from their conversion to their update, which read them again
+// from L2 before (256^3: 7x7 0.815 -> 0.796 ms, 15x7 0.873 -> 0.825, 8x8 0.940 ->
+// 0.890; in FP64, where they are registers, 15x5 1.407 -> 1.469 and not done),
+// and 16- and 32-wide rings, whose x faces go through shuffles, have no x
+// exchange buffers.
+template <typename T, typename V, int TXO, int TYO, int NQ = 2, bool KEEP = false> struct Geo {
   static constexpr int CX = 2 * TXO, CY = 2 * TYO;
   static constexpr int RW = CX + 2, RH = CY + 2;  // ring columns
   static constexpr int NRC = RW * RH;
@@ -75,8 +81,10 @@ template <typename T, typename V, int TXO, int TYO, int NQ = 2> struct Geo {
   static constexpr size_t kStageF = (size_t)NSTAGE * NSLOT * Store<T>::kSlotF * sizeof(float);
   static constexpr size_t kQ = (size_t)NQ * 5 * NLC * sizeof(V);
   static constexpr int kNQ = NQ;  // plane-buffer slot of plane (layer) p >= -2: RH_QSLOT(G, p)
-  static constexpr size_t kFS = (size_t)10 * NRC * sizeof(V);
-  static constexpr size_t kFX = (size_t)2 * 5 * NRC * sizeof(V);
+  static constexpr int kXBuf = KEEP && (RW == 16 || RW == 32) ? 0 : 5 * NRC;  // entries of an x exchange buffer
+  static constexpr size_t kFS = (size_t)(kXBuf + 5 * NRC) * sizeof(V);
+  static constexpr size_t kFX = (size_t)(kXBuf + 5 * NRC) * sizeof(V);
+  static constexpr size_t kU = KEEP ? (size_t)2 * NRC * 48 : 0;
   static constexpr size_t kRed = (size_t)NWARP * 4 * sizeof(double);
   static constexpr size_t kAmr = (size_t)NRC * (sizeof(int) + sizeof(uint32_t));
   static constexpr size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -88,7 +96,8 @@ template <typename T, typename V, int TXO, int TYO, int NQ = 2> struct Geo {
   static constexpr size_t oRed = a16(oFX + kFX);
   static constexpr size_t oAmr = a16(oRed + kRed);
   static constexpr int kRing = 8;  // table rows AsyncStager keeps: the update's to the one ahead of its copies, 6 at most
-  static constexpr size_t oRing = a16(oAmr + kAmr);
+  static constexpr size_t oU = a16(oAmr + kAmr);
+  static constexpr size_t oRing = a16(oU + kU);
   static constexpr size_t oBar = a16(oRing + (sizeof(T) == 4 ? (size_t)kRing * NSLOT * sizeof(int) : 0));
   static constexpr size_t kSmem = oBar + 64;
 };

@@ -14,6 +14,8 @@
 // Plane 2K is finished in the same iteration; plane 2K+1 waits one iteration
 // for the flux through face 2K+3/2.
 #pragma once
+#include <type_traits>
+
 #include "rh_godunov.cuh"
 
 namespace rh {
@@ -77,6 +79,15 @@ __device__ __forceinline__ void amr_face_f32(const LevelArgs& A, const StateArgs
     }
   }
 }
+
+// Shared-memory layout of the grid kernel (slope_type 3 needs the space of the
+// kept values for its third primitive layer) and of the batch kernel (whose
+// plane body needs the x exchange buffers of every tile: with the kept values
+// beside them two CTAs of 16-wide rings would not fit an SM).
+template <int TXO, int TYO, int SLOPE>
+using GridGeo2 = Geo<float, float2, TXO, TYO, (SLOPE == 3 ? 3 : 2), (SLOPE != 3)>;
+template <int TXO, int TYO>
+using BatchGeo2 = Geo<float, float2, TXO, TYO, 2, (2 * TXO + 2 != 16 && 2 * TXO + 2 != 32)>;
 
 // One pencil of the FP32-bulk step for a persistent CTA (as pencil_body_f64).
 template <int TXO, int TYO, int SLOPE, int RIEMANN, bool AMR, bool DENSE, class Sink>

@@ -40,7 +40,7 @@ cudaError_t launch_f64(const LevelArgs& A, const void* S, const void* H, int nbl
 
 template <int TXO, int TYO, int MINB, int SLOPE, int RIEMANN, bool AMR>
 cudaError_t launch_f32x2(const LevelArgs& A, const void* S, const void* H, int nblocks, cudaStream_t st) {
-  using G = Geo<float, float2, TXO, TYO, (SLOPE == 3 ? 3 : 2)>;
+  using G = GridGeo2<TXO, TYO, SLOPE>;
   auto k = godunov_pencil2_kernel<TXO, TYO, MINB, SLOPE, RIEMANN, AMR>;
   static bool attr = false;
   if (!attr) {
@@ -67,7 +67,7 @@ template <typename T, int TXO, int TYO, int MINB, bool AMR = false> struct TileR
     } else {
 #define RH_REG(S, R)                                                                                              \
   register_launcher({RH_PREC_FP32_BULK, TXO, TYO, MINB, S, R, AMR}, &launch_f32x2<TXO, TYO, MINB, S, R, AMR>,   \
-                    Geo<float, float2, TXO, TYO, (S == 3 ? 3 : 2)>::kSmem, Geo<float, float2, TXO, TYO>::NT);
+                    GridGeo2<TXO, TYO, S>::kSmem, Geo<float, float2, TXO, TYO>::NT);
       RH_REG(0, 1) RH_REG(0, 2) RH_REG(0, 3)
       RH_REG(1, 1) RH_REG(1, 2) RH_REG(1, 3)
       RH_REG(2, 1) RH_REG(2, 2) RH_REG(2, 3)

@@ -24,9 +24,9 @@ struct TileRate {
 const TileRate kRates[] = {
     {RH_PREC_FP64, 6, 4, 2, 12.7, {4.76, 6.01}},       {RH_PREC_FP64, 8, 4, 2, 12.6, {5.51, 6.82}},
     {RH_PREC_FP64, 8, 8, 1, 13.8, {7.00, 7.00}},       {RH_PREC_FP64, 7, 11, 1, 12.8, {6.88, 6.88}},
-    {RH_PREC_FP64, 15, 5, 1, 13.1, {6.71, 6.71}},      {RH_PREC_FP32_BULK, 6, 4, 2, 12.5, {2.56, 3.44}},
-    {RH_PREC_FP32_BULK, 8, 4, 2, 12.2, {3.08, 3.89}},  {RH_PREC_FP32_BULK, 7, 7, 2, 12.6, {3.20, 4.99}},
-    {RH_PREC_FP32_BULK, 8, 8, 1, 13.6, {3.88, 3.88}},  {RH_PREC_FP32_BULK, 15, 7, 1, 14.2, {5.45, 5.45}},
+    {RH_PREC_FP64, 15, 5, 1, 13.1, {6.71, 6.71}},      {RH_PREC_FP32_BULK, 6, 4, 2, 13.8, {2.45, 3.29}},
+    {RH_PREC_FP32_BULK, 8, 4, 2, 13.8, {2.92, 3.78}},  {RH_PREC_FP32_BULK, 7, 7, 2, 14.4, {3.12, 4.93}},
+    {RH_PREC_FP32_BULK, 8, 8, 1, 15.1, {3.67, 3.67}},  {RH_PREC_FP32_BULK, 15, 7, 1, 16.0, {5.18, 5.18}},
 };
 constexpr double kLaunch = 2.0;  // us of start that later waves of a launch do not pay
 constexpr int kMaxDepth = 48;    // layers; longer pencils only lost to the wave count
