@@ -22,10 +22,12 @@ extern "C" {
  * them): the new state and dt are the same bit for bit whatever the tile. */
 int rh_set_tile(int txo, int tyo, int minb, int lz);
 /* Tile of the coarse-fine (multi-level) kernels; before rh_set_mesh, since a
- * mesh's interpolated ghost octs follow its pencils.  Default (the fastest on
- * the AMR Sedov of levels 7-10): 7x7 octs, 2 CTAs/SM, 32 layers for FP32-bulk;
- * 8x4, 2 CTAs/SM, 32 layers for FP64.  rh_set_mesh gives a partial level
- * fewer layers (halved, down to 2) until its pencils fill a wave of CTAs. */
+ * mesh's interpolated ghost octs follow its pencils.  Default: 7x7 octs, 2
+ * CTAs/SM, 32 layers for FP32-bulk; 7x11, 1 CTA/SM, 32 layers for FP64.
+ * rh_set_mesh gives a partial level fewer layers (halved, down to 2) until its
+ * pencils fill a wave of CTAs, and, where this call did not choose the tile, a
+ * complete level fewer (halved, down to 4) while a pencil's march is longer
+ * than the whole mesh's work. */
 int rh_set_amr_tile(int txo, int tyo, int minb, int lz);
 int rh_get_tile(int* txo, int* tyo, int* minb, int* lz);
 /* Compiled tile shapes of a precision mode; returns their count. */

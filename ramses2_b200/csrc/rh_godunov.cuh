@@ -6,17 +6,19 @@
 //   * the pencil's oct table lists, for each of the L+2 layers (one halo layer
 //     each side) and each of the (TXO+2)(TYO+2) oct columns, the index of the
 //     oct whose cells fill that position (boundary sources already resolved);
-//   * each layer's oct records are staged into shared memory by bulk async
-//     copies (cp.async.bulk, one oct record per copy, completion counted on an
-//     mbarrier), two layers in flight, so the gather through the oct table runs
-//     ahead of the arithmetic;
+//   * each layer's oct records are staged into shared memory ahead of their
+//     conversion, by bulk async copies (Stager: cp.async.bulk, one oct record per
+//     copy, completion counted on an mbarrier, two layers in flight) or in the
+//     FP32-bulk grid kernels by 16-byte copies of all threads (AsyncStager), so
+//     the gather through the oct table runs ahead of the arithmetic;
 //   * one thread per "ring" cell column ((2TXO+2) x (2TYO+2) columns) converts
 //     its cells to primitive variables (ctoprim), keeps z-neighbours in
 //     registers, takes x/y neighbours from a shared plane buffer and computes
 //     slopes, the normal-velocity bound and the Hancock predictor (uslope +
 //     trace3d);
-//   * x/y interface states are exchanged through shared memory, z interface
-//     states never leave the thread; the Riemann fluxes of the three
+//   * y interface states are exchanged through shared memory, x ones too or (ring
+//     rows inside warps) through shuffles, z interface states never leave the
+//     thread; the Riemann fluxes of the three
 //     directions (cmpflxm + llf/hll/hllc) and the conservative update of the
 //     oct cells (godunov_fine.f90:733-816: x, then y, then z differences)
 //     follow;
