@@ -193,17 +193,16 @@ int upload_amr_tables(int l) {
   RH_CUDA(cudaMalloc(&T.d_ptab, sizeof(int) * std::max<size_t>(1, T.ptab.size())));
   RH_CUDA(cudaMalloc(&T.d_cfl_partial, sizeof(double) * 5 * std::max(1, T.npencil)));
   if (!T.phdr.empty()) {
-    RH_CUDA(cudaMemcpy(T.d_phdr, T.phdr.data(), sizeof(int4) * T.phdr.size(), cudaMemcpyHostToDevice));
-    RH_CUDA(cudaMemcpy(T.d_poff, T.poff.data(), sizeof(long long) * T.poff.size(), cudaMemcpyHostToDevice));
-    RH_CUDA(cudaMemcpy(T.d_ptab, T.ptab.data(), sizeof(int) * T.ptab.size(), cudaMemcpyHostToDevice));
+    RH_CUDA(copy_in(T.d_phdr, T.phdr.data(), sizeof(int4) * T.phdr.size()));
+    RH_CUDA(copy_in(T.d_poff, T.poff.data(), sizeof(long long) * T.poff.size()));
+    RH_CUDA(copy_in(T.d_ptab, T.ptab.data(), sizeof(int) * T.ptab.size()));
   }
   if (T.nghost > 0) {
     RH_CUDA(cudaMalloc(&T.d_gsrc_oct, sizeof(int) * T.gsrc_oct.size()));
     RH_CUDA(cudaMalloc(&T.d_gsrc_cf, T.gsrc_cf.size()));
-    RH_CUDA(cudaMemcpy(T.d_gsrc_oct, T.gsrc_oct.data(), sizeof(int) * T.gsrc_oct.size(), cudaMemcpyHostToDevice));
-    RH_CUDA(cudaMemcpy(T.d_gsrc_cf, T.gsrc_cf.data(), T.gsrc_cf.size(), cudaMemcpyHostToDevice));
-    RH_CUDA(cudaMemcpy(c.d_gfather + (T.gbase - c.ngridmax), T.gfather.data(), sizeof(int2) * T.gfather.size(),
-                       cudaMemcpyHostToDevice));
+    RH_CUDA(copy_in(T.d_gsrc_oct, T.gsrc_oct.data(), sizeof(int) * T.gsrc_oct.size()));
+    RH_CUDA(copy_in(T.d_gsrc_cf, T.gsrc_cf.data(), T.gsrc_cf.size()));
+    RH_CUDA(copy_in(c.d_gfather + (T.gbase - c.ngridmax), T.gfather.data(), sizeof(int2) * T.gfather.size()));
   }
   T.built = true;
   return RH_OK;

@@ -126,6 +126,17 @@ int stage64(long long noct, double** out) {
   *out = c.d_stage64;
   return RH_OK;
 }
+cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+  const cudaStream_t st = ctx().stream;
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+cudaError_t zero_in(void* dst, size_t bytes) {
+  const cudaStream_t st = ctx().stream;
+  const cudaError_t e = cudaMemsetAsync(dst, 0, bytes, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 template <typename E> __global__ void copy_kernel(E* __restrict__ dst, const E* __restrict__ src, long long n) {
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -386,7 +397,7 @@ int rh_init(int device_ordinal) {
   c.sm_count = prop.multiProcessorCount;
   RH_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
   RH_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
-  RH_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+  RH_CUDA(zero_in(c.d_err, sizeof(int)));
   RH_CUDA(cudaEventCreate(&c.ev0));
   RH_CUDA(cudaEventCreate(&c.ev1));
   RH_CUDA(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
@@ -436,7 +447,7 @@ int rh_sync(void) {
   int err = 0;
   RH_CUDA(cudaMemcpy(&err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
-    cudaMemset(c.d_err, 0, sizeof(int));
+    zero_in(c.d_err, sizeof(int));
     set_error("device wait bound exceeded (error word %d)", err);
     return RH_ETIMEDOUT;
   }
@@ -647,7 +658,7 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
       ref[i] = b;
     }
     RH_CUDA(cudaMalloc(&c.d_refmask, (size_t)n));
-    RH_CUDA(cudaMemcpy(c.d_refmask, ref.data(), (size_t)n, cudaMemcpyHostToDevice));
+    RH_CUDA(copy_in(c.d_refmask, ref.data(), (size_t)n));
     RH_CUDA(cudaMalloc(&c.d_gfather, sizeof(int2) * (size_t)std::max(1LL, nghost)));
     int nlev_ghost = 0;
     for (int l = c.levelmin; l <= c.levelmax; ++l) {

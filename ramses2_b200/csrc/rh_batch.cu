@@ -524,9 +524,9 @@ int rh_batch_init(int precision, int slope, int riemann, long long pool_octs) {
   RH_CUDA(cudaMalloc(&b.d_counter, sizeof(unsigned long long)));
   RH_CUDA(cudaMalloc(&b.d_bad, sizeof(int) * b.cap));
   RH_CUDA(cudaMalloc(&b.d_coff, sizeof(long long) * (b.cap + 1)));
-  RH_CUDA(cudaMemset(b.d_bad, 0, sizeof(int) * b.cap));
-  RH_CUDA(cudaMemset(b.d_counter, 0, sizeof(unsigned long long)));
-  RH_CUDA(cudaMemset(b.d_done, 0, sizeof(int) * b.cap));
+  RH_CUDA(zero_in(b.d_bad, sizeof(int) * b.cap));
+  RH_CUDA(zero_in(b.d_counter, sizeof(unsigned long long)));
+  RH_CUDA(zero_in(b.d_done, sizeof(int) * b.cap));
   b.probs.assign(b.cap, HostProb());
   b.free_list = {{0, pool_octs}};
   b.parity = 0;
@@ -681,7 +681,7 @@ int rh_batch_remove(int id) {
   free_octs(b.probs[id].oct0, b.probs[id].noct);
   b.probs[id] = HostProb();
   const int one = 1;
-  RH_CUDA(cudaMemcpy(b.d_done + id, &one, sizeof(int), cudaMemcpyHostToDevice));
+  RH_CUDA(copy_in(b.d_done + id, &one, sizeof(int)));
   b.dirty = true;
   return RH_OK;
 }
@@ -802,7 +802,7 @@ int rh_batch_poll(int* done, int* nstep, double* t) {
   RH_CUDA(cudaMemcpyAsync(&err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   RH_CUDA(cudaStreamSynchronize(c.stream));
   if (err) {
-    cudaMemset(c.d_err, 0, sizeof(int));
+    zero_in(c.d_err, sizeof(int));
     set_error("device wait bound exceeded in a batch step (error word %d)", err);
     return RH_ETIMEDOUT;
   }

@@ -78,7 +78,7 @@ int build_face_table(int l) {
   }
   if (c.d_face.size() < (size_t)c.levelmax + 1) c.d_face.resize(c.levelmax + 1, nullptr);
   RH_CUDA(cudaMalloc(&c.d_face[l], sizeof(int2) * std::max<size_t>(1, tab.size())));
-  RH_CUDA(cudaMemcpy(c.d_face[l], tab.data(), sizeof(int2) * tab.size(), cudaMemcpyHostToDevice));
+  RH_CUDA(copy_in(c.d_face[l], tab.data(), sizeof(int2) * tab.size()));
   return RH_OK;
 }
 

@@ -186,8 +186,8 @@ int build_sched(int l, HostStepSched& S) {
   RH_CUDA(cudaMalloc(&S.d_phdr, sizeof(int4) * std::max(1, S.npencil)));
   RH_CUDA(cudaMalloc(&S.d_poff, sizeof(long long) * std::max(1, S.npencil)));
   RH_CUDA(cudaMalloc(&S.d_partial, sizeof(double) * 5 * std::max(1, S.npencil)));
-  RH_CUDA(cudaMemcpy(S.d_phdr, ph.data(), sizeof(int4) * S.npencil, cudaMemcpyHostToDevice));
-  RH_CUDA(cudaMemcpy(S.d_poff, po.data(), sizeof(long long) * S.npencil, cudaMemcpyHostToDevice));
+  RH_CUDA(copy_in(S.d_phdr, ph.data(), sizeof(int4) * S.npencil));
+  RH_CUDA(copy_in(S.d_poff, po.data(), sizeof(long long) * S.npencil));
   RH_CUDA(cudaStreamCreateWithFlags(&S.up, cudaStreamNonBlocking));
   RH_CUDA(cudaStreamCreateWithFlags(&S.down, cudaStreamNonBlocking));
   RH_CUDA(cudaStreamCreateWithFlags(&S.unpk, cudaStreamNonBlocking));
@@ -369,7 +369,7 @@ int rh_coarse_step_host(const rh_hydro_params* p, const double* host_in, double*
   int err = 0;
   RH_CUDA(cudaMemcpy(&err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
-    cudaMemset(c.d_err, 0, sizeof(int));
+    zero_in(c.d_err, sizeof(int));
     set_error("device wait bound exceeded in a pencil kernel (error word %d)", err);
     return RH_ETIMEDOUT;
   }

@@ -199,6 +199,13 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
                  int slope, int riemann, const double* g, bool fuse_cfl, bool accumulate = false,
                  const PencilRange* range = nullptr, const LevelSlots* slots = nullptr);
 int stage64(long long noct, double** out);
+// Bytes of the host, or zeros, in device memory: there when these return, for
+// every stream.  (cudaMemcpy may return before bytes of pageable memory have
+// reached the device, cudaMemset does, and the library's non-blocking streams
+// do not wait for the default stream, where both run: a kernel launched next
+// can read what the memory held before.)
+cudaError_t copy_in(void* dst, const void* src, size_t bytes);
+cudaError_t zero_in(void* dst, size_t bytes);
 int ensure_level_tables(int l);
 TileCfg level_cfg(int l);  // tile of level l's launches (see rh_api.cu)
 // rh_tile.cu: tile and depth of a uniform level of nxo x nyo x nzo octs

@@ -49,7 +49,7 @@ int build_fathers() {
     }
   }
   RH_CUDA(cudaMalloc(&c.d_father, sizeof(int2) * fa.size()));
-  RH_CUDA(cudaMemcpy(c.d_father, fa.data(), sizeof(int2) * fa.size(), cudaMemcpyHostToDevice));
+  RH_CUDA(copy_in(c.d_father, fa.data(), sizeof(int2) * fa.size()));
   return RH_OK;
 }
 
