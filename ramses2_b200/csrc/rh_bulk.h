@@ -2,9 +2,10 @@
 //
 // One oct of FP32-bulk state is one 192-byte record: rho, rho u, rho v, rho w
 // of its 8 cells as float32 (cell fastest), then E of its 8 cells as float64.
-// A state buffer holds the records back to back, so one bulk copy stages an
-// oct.  Its float view uf and its double view ud (the buffer's doubles
-// advanced by kBulkE, i.e. the first record's E) index oct o's values as
+// A state buffer holds the records back to back, so one bulk copy, or twelve
+// 16-byte pieces, stage an oct.  Its float view uf and its double view ud (the
+// buffer's doubles advanced by kBulkE, i.e. the first record's E) index oct o's
+// values as
 // uf[o * kBulkF + 8 * var + cell] and ud[o * kBulkD + cell].
 #pragma once
 
