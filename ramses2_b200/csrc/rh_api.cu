@@ -432,6 +432,7 @@ int rh_finalize(void) {
   cudaEventDestroy(c.ev_cfl_ready);
   cudaStreamDestroy(c.cfl_copy);
   cudaFreeHost(c.h_cfl_next);
+  cudaFreeHost(c.h_cfl_own);
   cudaFreeHost(c.h_cfl_seq);
   for (auto s : c.lev_stream) cudaStreamDestroy(s);
   cudaStreamDestroy(c.stream);
@@ -645,6 +646,9 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   cudaFreeHost(c.h_cfl_next);
   c.h_cfl_next = nullptr;
   RH_CUDA(cudaMallocHost(&c.h_cfl_next, sizeof(double) * 5 * (c.levelmax + 1)));
+  cudaFreeHost(c.h_cfl_own);
+  c.h_cfl_own = nullptr;
+  RH_CUDA(cudaMallocHost(&c.h_cfl_own, sizeof(double) * 5 * (c.levelmax + 1)));
   cudaFreeHost(c.h_cfl_seq);
   c.h_cfl_seq = nullptr;
   RH_CUDA(cudaMallocHost(&c.h_cfl_seq, sizeof(unsigned long long) * (c.levelmax + 1)));
@@ -824,7 +828,7 @@ int rh_set_uold(int head_idx, int num_octs) {
 
 }  // extern "C"
 
-// Waits for the values that level l's last launch leaves in h_cfl_next (call
+// Waits for the values that level l's last launch leaves in h_cfl_own (call
 // with cfl_seq_of[l] != 0).  The host sees them as they are written, without
 // the end of the kernel, an event and a copy in between (steps of 16^3 FP32-bulk
 // 22.5 -> 20.5 us, of 64^3 FP64 48.3 -> 45.8); after 5 ms it waits for the stream, which also reports a failed kernel.
@@ -937,7 +941,7 @@ int rh_cmpdt(int head_idx, int num_octs, double dx, double gamma, double smallr,
         k[5] == (g ? g[0] : 0.0) && k[6] == (g ? g[1] : 0.0) && k[7] == (g ? g[2] : 0.0)) {
       RH_CUDA(cudaStreamSynchronize(c.stream));
       if (*(volatile unsigned long long*)(c.h_cfl_seq + lev) == c.cfl_seq_of[lev]) {
-        const double* v = c.h_cfl_next + 5 * lev;
+        const double* v = c.h_cfl_own + 5 * lev;
         *mass = v[0];
         *ekin = v[1];
         *eint = v[2];
@@ -1239,7 +1243,7 @@ int launch_level(int l, double gamma, double smallr, double smallc, double dt, d
   const bool reduce = fuse_cfl && !range && !(slots && slots->defer_reduce);
   A.ticket = reduce ? c.d_ticket + l : nullptr;
   A.cfl_out = c.d_cfl + 5 * l;
-  A.cfl_host = c.h_cfl_next + 5 * l;
+  A.cfl_host = c.h_cfl_own + 5 * l;
   A.seq_host = c.h_cfl_seq + l;
   A.seq = c.cfl_seq + 1;
   A.refmask = c.d_refmask;
@@ -1517,7 +1521,7 @@ int rh_coarse_step(const rh_hydro_params* p, double* dt, double* cfl) {
     const int l0 = lev.empty() ? 0 : lev.front(), nl = lev.empty() ? 0 : lev.back() - l0 + 1;
     if (all_cached && lev.size() == 1 && c.cfl_seq_of[l0]) {
       if ((rc = wait_cfl(l0))) return rc;
-      std::copy(c.h_cfl_next + 5 * l0, c.h_cfl_next + 5 * l0 + 5, h + 5 * l0);
+      std::copy(c.h_cfl_own + 5 * l0, c.h_cfl_own + 5 * l0 + 5, h + 5 * l0);
     } else if (all_cached && c.cfl_next_gen == c.cfl_gen && c.cfl_next_l0 == l0 && c.cfl_next_l1 == lev.back()) {
       // copied by the previous call as soon as they were final: no wait
       // for the rest of that step (its restrictions)

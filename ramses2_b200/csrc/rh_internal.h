@@ -106,8 +106,13 @@ struct Context {
   unsigned long long cfl_gen = 0, cfl_next_gen = ~0ull;
   double* h_cfl_next = nullptr;   // pinned, 5 per level
   // A launch that reduces its own partials (LevelArgs::ticket) stores the
-  // level's values there and then its number in h_cfl_seq; cfl_seq_of is the
-  // number whose values are the level's current ones (0: they came otherwise).
+  // level's values in h_cfl_own and then its number in h_cfl_seq; cfl_seq_of is
+  // the number whose values are the level's current ones (0: they came
+  // otherwise).  Slots of their own: no launch waits for the copy on cfl_copy,
+  // which may land in h_cfl_next after a later launch has stored its values.
+  // (It may also read d_cfl while that launch writes it; the launch bumped
+  // cfl_gen, so what it copied is not used.)
+  double* h_cfl_own = nullptr;    // pinned, 5 per level
   unsigned long long* h_cfl_seq = nullptr;  // pinned, one per level
   unsigned long long cfl_seq = 0;
   std::vector<unsigned long long> cfl_seq_of;
