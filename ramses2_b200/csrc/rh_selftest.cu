@@ -4,7 +4,7 @@
 //    word and the kernel returns; the host sees RH_ETIMEDOUT and the context
 //    stays usable.  No fault, trap or hang;
 //  * the FP64 lane reciprocal and square root of the pencil kernels (vrcp,
-//    vsqrt: hardware estimates refined by a third-order iteration) next to
+//    vsqrt: hardware estimates refined to rounding error) next to
 //    CUDA's correctly rounded 1.0/x and sqrt(x), element by element.
 #include <cuda_runtime.h>
 
