@@ -157,20 +157,21 @@ __global__ void cmpdt_kernel(const double* __restrict__ ud, const float* __restr
     const bool ref = refined ? refined[cell_id] != 0 : (refbits ? ((refbits[oct] >> cell) & 1) != 0 : false);
     if (!ref) {
       // in the fused epilogue's form, so that a level's values do not depend
-      // on which of the two computed them
+      // on which of the two computed them; a cell without a signal speed (no
+      // pressure at rest, or NaN) takes the longest step, as in cmpdt
       CflAcc a;
       if (!fp32) {
         const double* o = ud + oct * 40 + cell;
-        a.add(o[0], o[8], o[16], o[24], o[32], C);
+        a.add<true>(o[0], o[8], o[16], o[24], o[32], C);
       } else {
         const float* o = uf + oct * kBulkF + cell;
-        a.add(o[0], o[8], o[16], o[24], ud[oct * kBulkD + cell], C);
+        a.add<true>(o[0], o[8], o[16], o[24], ud[oct * kBulkD + cell], C);
       }
       a.scale(vol);
       m = a.mass;
       ek = a.ekin;
       ei = a.eint;
-      dt = a.dt(C);
+      dt = a.cmax > 0.0 ? a.dt(C) : C.cdx_smallc;
     }
   }
   for (int off = 16; off > 0; off >>= 1) {

@@ -239,21 +239,30 @@ constexpr long long kWaitBound = 1ll << 22;  // bounded mbarrier spin (seconds a
 // velocities and scaling each term by the volume took about 60.
 struct CflAcc {
   double mass = 0, ekin = 0, eint = 0, cmax = 0;
+  // positive, neither subnormal nor above 2^1022 (whose reciprocal is subnormal)
+  static __device__ __forceinline__ bool normal(double x) {
+    const int hi = __double2hiint(x);
+    return hi >= 0x00100000 && hi < 0x7fd00000;
+  }
   __device__ __forceinline__ void add(double r, double m1, double m2, double m3, double E, const LevelArgs& A) {
     add(r, m1, m2, m3, E, A.cfl);
   }
   // (an FP32-bulk cell's density and momenta widen exactly)
+  // ANY: arguments outside the normal numbers too (vrcp and vsqrt give NaN for
+  // a zero, subnormal or infinite one), by the IEEE operations there.
+  template <bool ANY = false>
   __device__ __forceinline__ void add(double r, double m1, double m2, double m3, double E, const CflConst& C) {
     mass += r;
     ekin += E;
     const double rm = r > C.smallr ? r : C.smallr;
-    const double irm = vrcp(rm);
+    const double irm = ANY && !normal(rm) ? 1.0 / rm : vrcp(rm);
     const double e = fma(-0.5 * fma(m1, m1, fma(m2, m2, m3 * m3)), irm, E);
     eint += e;
     double p = C.gm1 * e;
     const double pf = rm * C.smallp;
     p = p > pf ? p : pf;
-    const double c = vsqrt(C.gamma * p * irm);
+    const double c2 = C.gamma * p * irm;
+    const double c = ANY && !normal(c2) ? sqrt(c2) : vsqrt(c2);
     double a = fabs(m1);
     if (C.ndim > 1) a += fabs(m2);
     if (C.ndim > 2) a += fabs(m3);
