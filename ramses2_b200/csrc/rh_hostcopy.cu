@@ -15,8 +15,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 
 #include "rh_internal.h"
@@ -28,7 +29,8 @@ constexpr int kSlots = 12;  // on 16 cores 622 MB took 119 ms with 1, 50 with 4,
 constexpr long long kSlotOcts = 13056;  // 4.2 MB of FP64 oct records
 constexpr long long kPieceOcts = 1632;  // smallest piece, 522 KB
 constexpr size_t kSlotBytes = sizeof(double) * 40 * kSlotOcts;
-// Below this a plain copy is done before the workers have started.
+// Below this a plain copy is done before the workers have started, and nothing
+// is pinned for it.
 constexpr long long kMinOcts = kPieceOcts;
 
 struct Ring {
@@ -62,10 +64,24 @@ cudaError_t to_slot(Ring& r, int w, const OctSource& s, long long o, long long n
   return cudaGetLastError();
 }
 
-// Slots and streams, on the first large transfer.  Fewer than kSlots (even
-// none) where pinned memory is short.
-int ring_ready(Ring& r) {
-  while (r.n < kSlots) {
+// The calling thread's device, put back at the end of a transfer.
+struct DeviceScope {
+  int was = -1;
+  cudaError_t set(int device) {
+    cudaError_t e = cudaGetDevice(&was);
+    if (e != cudaSuccess) was = -1;
+    return e == cudaSuccess ? cudaSetDevice(device) : e;
+  }
+  ~DeviceScope() {
+    if (was >= 0) cudaSetDevice(was);
+  }
+};
+
+// Slots and streams for up to want workers, on the current device, kept for the
+// next transfers: pinning one takes 3 to 6 ms, so a transfer gets no more than
+// it has pieces.  Fewer (even none) where pinned memory is short.
+int ring_ready(Ring& r, int want) {
+  while (r.n < want) {
     if (!r.slot[r.n] && cudaMallocHost(&r.slot[r.n], kSlotBytes) != cudaSuccess) {
       r.slot[r.n] = nullptr;
       break;
@@ -74,22 +90,28 @@ int ring_ready(Ring& r) {
     ++r.n;
   }
   (void)cudaGetLastError();
-  return r.n;
+  return std::min(r.n, want);
 }
 
-// Without pinned memory: a plain copy, FP32-bulk records widened on the host.
+// A plain copy, FP32-bulk records widened on the host: few octs, or no pinned
+// memory.
 int plain_copy(double* dst, const OctSource& s, long long noct) {
   if (!s.uf) {
     RH_CUDA(cudaMemcpy(dst, s.ud, sizeof(double) * 40 * noct, cudaMemcpyDeviceToHost));
     return RH_OK;
   }
-  alignas(8) float rec[64 * kBulkF];
-  for (long long o = 0; o < noct; o += 64) {
-    const int n = (int)std::min<long long>(64, noct - o);
-    RH_CUDA(cudaMemcpy(rec, s.uf + o * kBulkF, (size_t)kBulkBytes * n, cudaMemcpyDeviceToHost));
-    for (int i = 0; i < n; ++i) {
+  const long long step = std::min(noct, kMinOcts);
+  std::unique_ptr<float[]> rec(new (std::nothrow) float[step * kBulkF]);
+  if (!rec) {
+    set_error("no host memory to read a state back");
+    return RH_ENOMEM;
+  }
+  for (long long o = 0; o < noct; o += step) {
+    const long long n = std::min(step, noct - o);
+    RH_CUDA(cudaMemcpy(rec.get(), s.uf + o * kBulkF, (size_t)kBulkBytes * n, cudaMemcpyDeviceToHost));
+    for (long long i = 0; i < n; ++i) {
       for (int k = 0; k < 32; ++k) dst[(o + i) * 40 + k] = rec[i * kBulkF + k];
-      std::memcpy(dst + (o + i) * 40 + 32, rec + i * kBulkF + 32, 8 * sizeof(double));
+      std::memcpy(dst + (o + i) * 40 + 32, rec.get() + i * kBulkF + 32, 8 * sizeof(double));
     }
   }
   return RH_OK;
@@ -108,26 +130,27 @@ bool pageable(const void* p) {
 
 int octs_to_host(double* dst, const OctSource& s, long long noct, int device) {
   if (noct <= 0) return RH_OK;
+  DeviceScope scope;
+  RH_CUDA(scope.set(device));
   if (!s.uf && !pageable(dst)) {  // pinned already: the link's rate without a slot
     RH_CUDA(cudaMemcpy(dst, s.ud, sizeof(double) * 40 * noct, cudaMemcpyDeviceToHost));
     return RH_OK;
   }
   Ring& r = ring();
   std::lock_guard<std::mutex> lock(r.mu);
-  const int slots = noct < kMinOcts && !s.uf ? 0 : ring_ready(r);
-  if (slots == 0) return plain_copy(dst, s, noct);
   // pieces of a slot's size, smaller where a transfer would leave workers idle
   // (47 MB in 12 problems: 9.0 ms with whole slots, 6.4 so; 620 MB in 24: 39 ms,
   // 48 with pieces of 522 KB throughout)
   const long long piece = std::min(kSlotOcts, std::max(kPieceOcts, noct / 16));
   const long long npiece = (noct + piece - 1) / piece;
+  const int hw = std::max(1, (int)std::thread::hardware_concurrency() * 3 / 4);
+  const int nw = noct < kMinOcts ? 0 : ring_ready(r, (int)std::min<long long>(std::min(kSlots, hw), npiece));
+  if (nw == 0) return plain_copy(dst, s, noct);
   std::atomic<long long> next{0};
   std::atomic<int> err{cudaSuccess};
   auto work = [&](int w) {
-    if (const cudaError_t e = cudaSetDevice(device); e != cudaSuccess) {
-      if (w == 0) err = e;
-      return;  // another worker's pieces go to the caller, worker 0
-    }
+    // a worker without the device leaves its pieces to the caller, worker 0
+    if (w > 0 && cudaSetDevice(device) != cudaSuccess) return;
     for (long long i; (i = next.fetch_add(1)) < npiece;) {
       const long long o = i * piece, n = std::min(piece, noct - o);
       cudaError_t e = to_slot(r, w, s, o, n);
@@ -139,14 +162,12 @@ int octs_to_host(double* dst, const OctSource& s, long long noct, int device) {
       std::memcpy(dst + o * 40, r.slot[w], sizeof(double) * 40 * n);
     }
   };
-  const int hw = (int)std::thread::hardware_concurrency();
-  const int nw = (int)std::min<long long>(std::min(slots, std::max(1, hw * 3 / 4)), npiece);
   std::thread th[kSlots];
   for (int w = 1; w < nw; ++w) {
     try {
       th[w] = std::thread(work, w);
-    } catch (const std::system_error&) {
-      break;  // no more threads: the running ones take the pieces
+    } catch (...) {
+      break;  // no more threads, or memory for them: the running ones take the pieces
     }
   }
   work(0);

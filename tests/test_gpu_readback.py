@@ -68,3 +68,26 @@ def test_mesh_state_to_pageable_and_pinned_memory(prec):
         assert np.array_equal(out, want)
     finally:
         g.close()
+
+
+def resident_mb():
+    with open("/proc/self/status") as f:
+        return next(int(l.split()[1]) for l in f if l.startswith("VmRSS")) / 1024.0
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32_bulk"])
+def test_small_read_backs_pin_no_memory(prec):
+    """The pinned slots (4.2 MB each, kept until the library is closed) come with
+    the first transfer that needs them, as many as it has workers for."""
+    b = Batch(prec, pool_octs=1 << 16)
+    try:
+        small = b.add(problem((2, 2, 2), dx=1.0, max_steps=1), ic_host(octs(1, 0)))
+        two = b.add(problem((2, 2, 2 * 3264), dx=1.0, max_steps=1), ic_host(octs(3264, 1)))
+        b.status(small)
+        before = resident_mb()
+        assert np.array_equal(b.fetch(small), as_stored(octs(1, 0), prec))
+        assert resident_mb() - before < 2.0
+        assert np.array_equal(b.fetch(two), as_stored(octs(3264, 1), prec))
+        assert resident_mb() - before < 4 * 4.2  # two pieces of 1,632 octs: two slots and the result
+    finally:
+        b.close()
