@@ -63,7 +63,11 @@ int rh_batch_remove(int id);
 int rh_batch_step(int nsteps);
 /* Per-problem state: time, steps taken, done flag (0 running, 1 finished,
  * 2 stopped by the state check), current dt and the courant_fine totals
- * (mass, ekin, eint, emag, dt) of the current state. */
+ * (mass, ekin, eint, emag, dt) of the current state.  State, time, steps and dt
+ * do not depend on the other problems of the batch, bit for bit; the sums of
+ * mass, ekin and eint do not either once rh_batch_set_tile has chosen the tile,
+ * and to rounding before (their order follows the tile and depth, which follow
+ * the problems in the batch). */
 int rh_batch_status(int id, double* t, int* nstep, int* done, double* dt, double* totals5);
 /* Status of every problem slot at once (arrays of rh_batch_capacity()). */
 int rh_batch_poll(int* done, int* nstep, double* t);

@@ -110,3 +110,34 @@ def test_default_batch_depth_steps_like_an_explicit_one(prec, tile):
         assert (sa["t"], sa["dt"], sa["nstep"]) == (sb["t"], sb["dt"], sb["nstep"])
         assert sa["totals"] == pytest.approx(sb["totals"], rel=1e-12)
         assert np.array_equal(ua, ub)
+
+
+@pytest.mark.parametrize("tile", [(8, 4, 2, 32), None])
+@pytest.mark.parametrize("prec", ["fp64", "fp32_bulk"])
+def test_totals_and_the_neighbours(prec, tile):
+    """A problem alone and among others that change the default depth and (in
+    FP32-bulk, as 2D ones) tile, arriving in mid-run: its sums are the same with a
+    chosen tile and equal to rounding without."""
+    p = problem((48, 32, 64), dx=1 / 64, bc="outflow", max_steps=6)
+    ic = ic_blast([1.0, 0.1, 0.2, 0.0, 0.1], 5.0, 0.1, [0.3, 0.2, 0.5])
+    plane = problem((512, 512, 2), dx=1 / 512, ndim=2, bc=["outflow"] * 4 + ["periodic"] * 2, max_steps=20)
+    cube = problem((64, 64, 64), dx=1 / 64, bc="periodic", max_steps=20)
+    got = []
+    for others in ([], [plane, cube, cube]):
+        b = Batch(prec, pool_octs=1 << 19, tile=tile)
+        try:
+            pid = b.add(p, ic)
+            b.step(3)
+            for o in others:
+                b.add(o, ic)
+            b.step(3)
+            got.append((b.status(pid), b.fetch(pid)))
+        finally:
+            b.close()
+    (sa, ua), (sb, ub) = got
+    assert sa["nstep"] == sb["nstep"] == 6
+    assert (sa["t"], sa["dt"]) == (sb["t"], sb["dt"]) and np.array_equal(ua, ub)
+    if tile:
+        assert list(sa["totals"]) == list(sb["totals"])
+    else:  # another order of 98,304 positive terms
+        assert sa["totals"] == pytest.approx(sb["totals"], rel=1e-13)
