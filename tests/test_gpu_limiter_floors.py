@@ -5,7 +5,8 @@ The floors (smallr on the density, smallr*smallc**2 on the pressure of an
 interface state) sit behind one test per cell in the kernels; here they act in
 part of the cells (a floor inside the range of the states), in none, and next
 to zero.  The limiters see equal neighbours, differences of opposite sign and
-differences whose product underflows FP32."""
+(on a state whose momenta are compared on their own scale) differences whose
+product underflows FP32."""
 import os
 
 import numpy as np
@@ -76,3 +77,32 @@ def test_plateaus_and_tiny_differences(prec, amp):
     eps = 2.3e-16 if prec == "fp64" else 1.2e-7
     assert np.abs(out - ref).max() <= 8 * eps
     assert np.all(np.isfinite(out))
+
+
+@pytest.mark.parametrize("slope", [1, 2])
+@pytest.mark.parametrize("prec", ["fp64", "fp32_bulk"])
+def test_differences_whose_product_underflows(prec, slope):
+    """Velocities of some 1e-20 in a gas whose sound speed is 1e-18: every term
+    of the step is a normal FP32 number, but the product of two velocity
+    differences (1e-40) is not, so a limiter that tests its sign takes no slope.
+    The momenta change by 2 %, and by a third of that less without slopes."""
+    m = uniform_mesh(4, bc="periodic")
+    r = np.random.default_rng(8)
+    n, rho, p = 16, 1e15, 1e-21
+    x = 2 * np.pi * (np.arange(n) + 0.5) / n
+    wave = np.sin(x)[None, None, :] + np.sin(x)[None, :, None] + np.sin(x)[:, None, None]
+    v = 1e-20 * (wave + 0.3 * r.uniform(-1, 1, (3, n, n, n)))
+    one = np.ones((n, n, n))
+    u = prim_to_cons(rho * one, *v, p * one, 1.4)
+    m.from_dense(u, 4)
+    P = HydroParams.make(gamma=1.4, smallr=1e-10, smallc=1e-30, slope_type=slope, riemann="hllc")
+    dt = 0.1 * m.dx(4) / np.sqrt(1.4 * p / rho)
+    u0 = m.uold.copy()
+    ref, out = one_step(m, P, prec, (8, 4, 4), dt)
+    change = np.abs(ref - u0)[:, 1:4].max()
+    eps = 2.3e-16 if prec == "fp64" else 1.2e-7
+    # the momentum update is dt/dx times differences of fluxes p + rho u du of
+    # which p is the largest term: a few roundings of it, and of the momenta
+    bound = 8 * eps * (p * dt / m.dx(4) + np.abs(ref[:, 1:4]).max())
+    assert change > 1e3 * bound
+    assert np.abs(out - ref)[:, 1:4].max() <= bound
