@@ -67,7 +67,8 @@ template <> struct Store<float> {  // FP32-bulk: one 192-byte record per oct (rh
 // 0.890; in FP64, where they are registers, 15x5 1.407 -> 1.469 and not done),
 // and 16- and 32-wide rings, whose x faces go through shuffles, have no x
 // exchange buffers.
-template <typename T, typename V, int TXO, int TYO, int NQ = 2, bool KEEP = false> struct Geo {
+// RING: room for the table rows that AsyncStager keeps.
+template <typename T, typename V, int TXO, int TYO, int NQ = 2, bool KEEP = false, bool RING = false> struct Geo {
   static constexpr int CX = 2 * TXO, CY = 2 * TYO;
   static constexpr int RW = CX + 2, RH = CY + 2;  // ring columns
   static constexpr int NRC = RW * RH;
@@ -100,7 +101,7 @@ template <typename T, typename V, int TXO, int TYO, int NQ = 2, bool KEEP = fals
   static constexpr int kRing = 8;  // table rows AsyncStager keeps: the update's to the one ahead of its copies, 6 at most
   static constexpr size_t oU = a16(oAmr + kAmr);
   static constexpr size_t oRing = a16(oU + kU);
-  static constexpr size_t oBar = a16(oRing + (sizeof(T) == 4 ? (size_t)kRing * NSLOT * sizeof(int) : 0));
+  static constexpr size_t oBar = a16(oRing + (RING ? (size_t)kRing * NSLOT * sizeof(int) : 0));
   static constexpr size_t kSmem = oBar + 64;
 };
 

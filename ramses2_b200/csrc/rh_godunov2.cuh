@@ -85,7 +85,7 @@ __device__ __forceinline__ void amr_face_f32(const LevelArgs& A, const StateArgs
 // plane body needs the x exchange buffers of every tile: with the kept values
 // beside them two CTAs of 16-wide rings would not fit an SM).
 template <int TXO, int TYO, int SLOPE>
-using GridGeo2 = Geo<float, float2, TXO, TYO, (SLOPE == 3 ? 3 : 2), (SLOPE != 3)>;
+using GridGeo2 = Geo<float, float2, TXO, TYO, (SLOPE == 3 ? 3 : 2), (SLOPE != 3), true>;
 template <int TXO, int TYO>
 using BatchGeo2 = Geo<float, float2, TXO, TYO, 2, (2 * TXO + 2 != 16 && 2 * TXO + 2 != 32)>;
 
@@ -94,7 +94,6 @@ template <int TXO, int TYO, int SLOPE, int RIEMANN, bool AMR, bool DENSE, class 
 __device__ __forceinline__ void pencil_body_f32(const LevelArgs& A, const StateArgs<float>& S,
                                                 const HydroK<float2>& H, const int4 hdr, const int* tab, int rbase,
                                                 const Sink sink) {
-  constexpr bool init_barriers = false;
 #include "rh_pencil_f32.inc"
 }
 
@@ -103,7 +102,6 @@ template <int TXO, int TYO, int MINB, int SLOPE, int RIEMANN, bool AMR>
 __global__ void __launch_bounds__(Geo<float, float2, TXO, TYO>::NT, MINB)
 godunov_pencil2_kernel(const LevelArgs A, const StateArgs<float> S, const HydroK<float2> H) {
   constexpr bool DENSE = false;
-  constexpr bool init_barriers = true;
   constexpr int rbase = 0;
   const GridCflSink sink{};
   const int4 hdr = A.phdr[blockIdx.x];

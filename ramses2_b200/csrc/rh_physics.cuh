@@ -51,8 +51,8 @@ template <class V> __device__ __forceinline__ V momentum_bound(V dq, V rm1, V vm
 }
 
 
-// Half of limited_slope and of the momentum bound, for slope types 0-2, as
-// the predictor takes them.  Half the moncen slope is the minmod of a, b and
+// Half of the limited slope (umuscl.f90:2132-2206) and of the momentum bound,
+// for slope types 0-2, as the predictor takes them.  Half the moncen slope is the minmod of a, b and
 // (a + b)/4 (scaling by two commutes with rounding, so min(2|a|, 2|b|,
 // |a + b|/2)/2 is formed without the factors of two), half the minmod slope
 // half of that of a and b.
