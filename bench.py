@@ -849,7 +849,7 @@ def run_ours(args):
     value = world * ncell / (ms * 1e-3)
     kms = kernel_ms[prec]
     achieved = ncell * B_ALG[prec] / (kms * 1e-3) / 1e9
-    launches = args.steps * 2  # pencil kernel + partial reduction per step (rh_cmpdt hits the fused CFL)
+    launches = args.steps  # one pencil kernel a step: its last CTA reduces the level's courant_fine values
     line = {
         "metric": "cell-updates/s Sedov3D 256^3 FP32-bulk vs FP64 at L1<=1e-5; p50/p99 solve latency",
         "value": value,
@@ -900,10 +900,51 @@ def run_ours(args):
         "gpu_launches": launches,
         "clocks": results[prec]["clocks"],
     }
-    print(json.dumps(line))
+    if args.detail:
+        with open(args.detail, "w") as f:
+            json.dump(line, f, indent=1)
+    print(json.dumps(printed(line)))
     if dist is not None:
         dist.barrier()
         dist.destroy_process_group()
+
+
+LEGS = ("fp64", "sedov512_periodic", "amr", "turbulence", "batch", "serve", "snapshot")
+# of a leg: what its workload is and how it was measured, in the unabridged record
+LEG_DETAIL = {"workload", "unit", "clocks", "tile", "cells_all_levels", "octs_per_level", "check_every", "ms_each_step",
+              "all_level_cell_updates_per_s", "set_mesh_s", "pipes_ncu", "rejected", "served", "makespan_s",
+              "steps_min", "steps_max", "cell_updates", "mean_cell_updates_per_request", "rate_hz", "requests", "bytes",
+              "algorithmic_bytes", "steps"}
+
+
+def short(v, drop=()):
+    """The record as it is printed: numbers to six digits, a list of checks as
+    the largest error of each kind."""
+    if isinstance(v, float):
+        return float("%.6g" % v)
+    if isinstance(v, dict):
+        return {k: short(x, drop) for k, x in v.items() if k not in drop}
+    if not isinstance(v, list) or not v:
+        return v
+    if isinstance(v[0], dict) and ("rel_l1" in v[0] or "rho" in v[0] or "fp64" in v[0]):
+        worst = {}
+
+        def walk(d, key):
+            for k, x in d.items():
+                if isinstance(x, dict):
+                    walk(x, key if k == "rel_l1" else k + "_")
+                elif isinstance(x, float) and k != "dt_gpu":
+                    k = key + ("rel_l1_rho" if k == "rho" else "rel_l1_others" if k in ("mx", "my", "mz", "E") else k)
+                    worst[k] = max(worst.get(k, 0.0), x)
+
+        for c in v:
+            walk(c, "")
+        return short(dict({"checks": len(v)}, **worst))
+    return [short(x, drop) for x in v]
+
+
+def printed(line):
+    return {k: short(v, LEG_DETAIL if k in LEGS else ()) for k, v in line.items()}
 
 
 def run_reference(args):
@@ -966,6 +1007,7 @@ def main():
     ap.add_argument("--serve-rate", type=float, default=20.0, help="request arrivals per second")
     ap.add_argument("--serve-sweep-requests", type=int, default=100,
                     help="requests per point of the latency-vs-offered-load sweep (0: skip)")
+    ap.add_argument("--detail", default="", help="file for the unabridged record (every step time and check)")
     args = ap.parse_args()
     args.warmup = max(3, args.warmup)
     if args.impl == "reference":
