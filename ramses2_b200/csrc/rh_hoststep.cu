@@ -67,8 +67,11 @@ namespace {
 // Pencils this deep: a pencil needs its neighbourhood and a chunk waits for
 // the pencils that write it, so shallow pencils start earlier and release
 // chunks sooner; their extra halo work is hidden behind the copies.  Steps with
-// 2 and with 8 layers: 256^3 18.1 / 18.4 ms FP32-bulk, 17.8 / 18.3 FP64; 64^3
-// 0.46 / 0.47 and 0.46 / 0.49; 32^3 0.120 / 0.139 and 0.116 / 0.149.
+// 2 and with 8 layers: 256^3 FP32-bulk 17.8 / 18.2 ms; 64^3 0.457 / 0.474 FP32-bulk,
+// 0.454 / 0.483 FP64.  A 256^3 FP64 step takes 17.5 ms with 2 layers every time;
+// with 8 it takes 16.0 or 18.4 from one call to the next, by how the two copy
+// directions happen to share the link (means of 40 to 60 calls on 8x8 octs: 16.7
+// to 18.1 ms by box and process), so 2 are taken there too.
 constexpr int kSchedLz = 2;
 // 128 chunks of 16,384 octs (5.2 MB of FP64 state per copy) for a 256^3
 // level: on one box 18.8-18.9 ms per FP32-bulk step, against 18.3-19.6 with

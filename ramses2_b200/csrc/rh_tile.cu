@@ -2,14 +2,20 @@
 //
 // A CTA marches its pencil layer by layer, so a level's step takes the CTAs'
 // waves times a pencil's march: a 64^3 level cut into 8x8-octs x 32-layer
-// pencils is 16 CTAs on 148 SMs, each marching 34 layers (FP64 257 us), while
-// 256 pencils of 8x4 octs x 4 layers take 41 us; a 256^3 level fills the chip with either
+// pencils is 16 CTAs on 148 SMs, each marching 34 layers (FP64 240 us), while
+// 256 pencils of 8x4 octs x 4 layers take 43 us; a 256^3 level fills the chip with either
 // and wants the tile with the least halo.  choose_tile() evaluates that time
 // for the compiled tiles below and the depths that cut the level's layers
 // evenly, from three rates per tile measured on a B200 (HLLC, moncen; boxes of
 // 16^3 to 256^3 cells, even and uneven; launch gap included): with one CTA on
 // an SM or two, a pencil of L layers takes start + L * layer[0 or 1] us.  On
-// those boxes its choice is within 1 % of the fastest of all tiles and depths.
+// those boxes its choice is the fastest of these tiles and depths.  The slope
+// type and solver of a run are not known when its mesh is set: types 0 and 1
+// and the other solvers change all rates alike, slope_type 3 (1.8 times the
+// time; one CTA of FP32-bulk 7x7 on an SM) does not, and its runs are up to 15 %
+// from their fastest tile (256^3 FP32-bulk 1.45 ms, 15x7 1.26; FP64 2.51, 7x11
+// 2.40).  On 25 boxes no choice was slower than 8x8 octs x 32 layers for slope
+// types 0, 1 or 3.
 #include <algorithm>
 
 #include "rh_internal.h"
@@ -22,9 +28,9 @@ struct TileRate {
   double start, layer[2];
 };
 const TileRate kRates[] = {
-    {RH_PREC_FP64, 6, 4, 2, 12.7, {4.76, 6.01}},       {RH_PREC_FP64, 8, 4, 2, 12.6, {5.51, 6.82}},
-    {RH_PREC_FP64, 8, 8, 1, 13.8, {7.00, 7.00}},       {RH_PREC_FP64, 7, 11, 1, 12.8, {6.88, 6.88}},
-    {RH_PREC_FP64, 15, 5, 1, 13.1, {6.71, 6.71}},      {RH_PREC_FP32_BULK, 6, 4, 2, 13.8, {2.45, 3.29}},
+    {RH_PREC_FP64, 6, 4, 2, 14.5, {4.96, 6.22}},       {RH_PREC_FP64, 8, 4, 2, 14.4, {5.62, 6.95}},
+    {RH_PREC_FP64, 8, 8, 1, 15.2, {7.19, 7.19}},       {RH_PREC_FP64, 7, 11, 1, 14.7, {7.04, 7.04}},
+    {RH_PREC_FP64, 15, 5, 1, 15.1, {6.74, 6.74}},      {RH_PREC_FP32_BULK, 6, 4, 2, 13.8, {2.45, 3.29}},
     {RH_PREC_FP32_BULK, 8, 4, 2, 13.8, {2.92, 3.78}},  {RH_PREC_FP32_BULK, 7, 7, 2, 14.4, {3.12, 4.93}},
     {RH_PREC_FP32_BULK, 8, 8, 1, 15.1, {3.67, 3.67}},  {RH_PREC_FP32_BULK, 15, 7, 1, 16.0, {5.18, 5.18}},
 };

@@ -50,7 +50,8 @@ __device__ __forceinline__ double vrcp(double x) {
 // last rounding only.  Seven operations in a chain of five; two Newton-Raphson
 // steps on y0 and the Heron step took twelve.  (The binomial series to third
 // order without the Heron step is five, but 12.5 % of its results are a rounding
-// off, up to 0.75 ulp.)
+// off, up to 0.75 ulp.  Both in their shorter forms: a 256^3 FP64 step 1.407 ms,
+// 1.445 with these.)
 __device__ __forceinline__ double vsqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
