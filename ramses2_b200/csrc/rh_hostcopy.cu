@@ -29,14 +29,16 @@ constexpr int kSlots = 12;  // on 16 cores 622 MB took 119 ms with 1, 50 with 4,
 constexpr long long kSlotOcts = 13056;  // 4.2 MB of FP64 oct records
 constexpr long long kPieceOcts = 1632;  // smallest piece, 522 KB
 constexpr size_t kSlotBytes = sizeof(double) * 40 * kSlotOcts;
-// Below this a plain copy is done before the workers have started, and nothing
-// is pinned for it.
+// Below this a copy is done before the workers have started: FP64 a plain one,
+// FP32-bulk through a slot of its own, of one smallest piece (1,024 octs 55 us;
+// 88 when the host widens the records; all slots pinned for it: 34 ms once).
 constexpr long long kMinOcts = kPieceOcts;
+constexpr int kSmall = kSlots;  // index of that slot
 
 struct Ring {
   std::mutex mu;  // one transfer at a time
-  double* slot[kSlots] = {};
-  cudaStream_t stream[kSlots] = {};
+  double* slot[kSlots + 1] = {};
+  cudaStream_t stream[kSlots + 1] = {};
   int n = 0;
 };
 Ring& ring() {
@@ -77,24 +79,25 @@ struct DeviceScope {
   }
 };
 
-// Slots and streams for up to want workers, on the current device, kept for the
-// next transfers: pinning one takes 3 to 6 ms, so a transfer gets no more than
-// it has pieces.  Fewer (even none) where pinned memory is short.
-int ring_ready(Ring& r, int want) {
-  while (r.n < want) {
-    if (!r.slot[r.n] && cudaMallocHost(&r.slot[r.n], kSlotBytes) != cudaSuccess) {
-      r.slot[r.n] = nullptr;
-      break;
-    }
-    if (cudaStreamCreateWithFlags(&r.stream[r.n], cudaStreamNonBlocking) != cudaSuccess) break;
-    ++r.n;
-  }
+// Slot w of the given size and its stream, on the current device, kept for the
+// next transfers.  False where pinned memory is short.
+bool slot_ready(Ring& r, int w, size_t bytes) {
+  if (!r.slot[w] && cudaMallocHost(&r.slot[w], bytes) != cudaSuccess) r.slot[w] = nullptr;
+  if (r.slot[w] && !r.stream[w] && cudaStreamCreateWithFlags(&r.stream[w], cudaStreamNonBlocking) != cudaSuccess)
+    r.stream[w] = nullptr;
   (void)cudaGetLastError();
+  return r.slot[w] && r.stream[w];
+}
+
+// Slots for up to want workers: pinning one takes 3 to 6 ms, so a transfer gets
+// no more than it has pieces.
+int ring_ready(Ring& r, int want) {
+  while (r.n < want && slot_ready(r, r.n, kSlotBytes)) ++r.n;
   return std::min(r.n, want);
 }
 
-// A plain copy, FP32-bulk records widened on the host: few octs, or no pinned
-// memory.
+// A plain copy, FP32-bulk records widened on the host: few octs in FP64, or no
+// pinned memory.
 int plain_copy(double* dst, const OctSource& s, long long noct) {
   if (!s.uf) {
     RH_CUDA(cudaMemcpy(dst, s.ud, sizeof(double) * 40 * noct, cudaMemcpyDeviceToHost));
@@ -132,7 +135,10 @@ int octs_to_host(double* dst, const OctSource& s, long long noct, int device) {
   if (noct <= 0) return RH_OK;
   DeviceScope scope;
   RH_CUDA(scope.set(device));
-  if (!s.uf && !pageable(dst)) {  // pinned already: the link's rate without a slot
+  // pinned already: the link's rate without a slot (FP32-bulk goes through slots:
+  // a kernel storing to dst would need all of it pinned, and only its first byte
+  // is known to be)
+  if (!s.uf && !pageable(dst)) {
     RH_CUDA(cudaMemcpy(dst, s.ud, sizeof(double) * 40 * noct, cudaMemcpyDeviceToHost));
     return RH_OK;
   }
@@ -144,7 +150,14 @@ int octs_to_host(double* dst, const OctSource& s, long long noct, int device) {
   const long long piece = std::min(kSlotOcts, std::max(kPieceOcts, noct / 16));
   const long long npiece = (noct + piece - 1) / piece;
   const int hw = std::max(1, (int)std::thread::hardware_concurrency() * 3 / 4);
-  const int nw = noct < kMinOcts ? 0 : ring_ready(r, (int)std::min<long long>(std::min(kSlots, hw), npiece));
+  const bool few = noct < kMinOcts;
+  const int nw = few ? 0 : ring_ready(r, (int)std::min<long long>(std::min(kSlots, hw), npiece));
+  if (few && s.uf && slot_ready(r, kSmall, sizeof(double) * 40 * kMinOcts)) {
+    RH_CUDA(to_slot(r, kSmall, s, 0, noct));
+    RH_CUDA(cudaStreamSynchronize(r.stream[kSmall]));
+    std::memcpy(dst, r.slot[kSmall], sizeof(double) * 40 * noct);
+    return RH_OK;
+  }
   if (nw == 0) return plain_copy(dst, s, noct);
   std::atomic<long long> next{0};
   std::atomic<int> err{cudaSuccess};
@@ -180,8 +193,8 @@ int octs_to_host(double* dst, const OctSource& s, long long noct, int device) {
 void free_host_ring() {
   Ring& r = ring();
   std::lock_guard<std::mutex> lock(r.mu);
-  for (int w = 0; w < kSlots; ++w) {
-    if (w < r.n) cudaStreamDestroy(r.stream[w]);
+  for (int w = 0; w <= kSlots; ++w) {
+    if (r.stream[w]) cudaStreamDestroy(r.stream[w]);
     cudaFreeHost(r.slot[w]);
     r.slot[w] = nullptr;
     r.stream[w] = nullptr;

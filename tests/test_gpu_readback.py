@@ -76,9 +76,10 @@ def resident_mb():
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32_bulk"])
-def test_small_read_backs_pin_no_memory(prec):
+def test_small_read_backs_pin_little_memory(prec):
     """The pinned slots (4.2 MB each, kept until the library is closed) come with
-    the first transfer that needs them, as many as it has workers for."""
+    the first transfer that needs them, as many as it has workers for; a small
+    FP32-bulk one has a slot of 0.5 MB."""
     b = Batch(prec, pool_octs=1 << 16)
     try:
         small = b.add(problem((2, 2, 2), dx=1.0, max_steps=1), ic_host(octs(1, 0)))
@@ -86,8 +87,8 @@ def test_small_read_backs_pin_no_memory(prec):
         b.status(small)
         before = resident_mb()
         assert np.array_equal(b.fetch(small), as_stored(octs(1, 0), prec))
-        assert resident_mb() - before < 2.0
+        assert resident_mb() - before < 4.0  # less than one slot
         assert np.array_equal(b.fetch(two), as_stored(octs(3264, 1), prec))
-        assert resident_mb() - before < 4 * 4.2  # two pieces of 1,632 octs: two slots and the result
+        assert resident_mb() - before < 4.0 + 3 * 4.2  # two pieces of 1,632 octs: two slots and the result
     finally:
         b.close()
