@@ -23,7 +23,8 @@ extern "C" {
 int rh_set_tile(int txo, int tyo, int minb, int lz);
 /* Tile of the coarse-fine (multi-level) kernels; before rh_set_mesh, since a
  * mesh's interpolated ghost octs follow its pencils.  Default: 7x7 octs, 2
- * CTAs/SM, 32 layers for FP32-bulk; 7x11, 1 CTA/SM, 32 layers for FP64.
+ * CTAs/SM, 32 layers for FP32-bulk; for FP64 7x11, 1 CTA/SM, 32 layers, or 8x4, 2
+ * CTAs/SM, where the mesh's octs are so scattered that its smaller tiles cost less.
  * rh_set_mesh gives a partial level fewer layers (halved, down to 2) until its
  * pencils fill a wave of CTAs, and, where this call did not choose the tile, a
  * complete level fewer (halved, down to 4) while a pencil's march is longer

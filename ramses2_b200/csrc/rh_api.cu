@@ -525,9 +525,6 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   int rc = check_ready(false);
   if (rc) return rc;
   Context& c = ctx();
-  // coarse-fine tile unless chosen: the fastest on AMR Sedovs per precision
-  // (FP64 on levels 6-9: 7x11 0.52 ms a coarse step, 8x4 0.58, 15x5 0.60)
-  if (!c.amr_cfg_set) c.amr_cfg = c.precision == RH_PREC_FP32_BULK ? TileCfg{7, 7, 2, 32} : TileCfg{7, 11, 1, 32};
   if (!m || !uold || !m->grid || !m->head || !m->noct) {
     set_error("rh_set_mesh: null pointer");
     return RH_EINVAL;
@@ -581,6 +578,11 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
       c.cfg = choose_tile(c.precision, (int)nx, (int)ny, (int)nz, c.sm_count);
   }
   c.levels.assign(c.levelmax + 1, LevelTables());
+  for (int l = c.levelmin; l <= c.levelmax; ++l)
+    c.levels[l].complete_box = c.noct[l] > 0 && (long long)c.noct[l] == ((long long)c.box_nx[0] << (l - 1)) *
+                                                                            ((long long)c.box_nx[1] << (l - 1)) *
+                                                                            ((long long)c.box_nx[2] << (l - 1));
+  if (!c.amr_cfg_set) c.amr_cfg = choose_amr_tile(c);
   // coarse-fine levels: tables first, they fix the number of ghost octs
   long long nghost = 0;
   std::vector<std::pair<int2*, long long>> dev_gfather;  // device-built ghost fathers, per level
@@ -593,9 +595,6 @@ int rh_set_mesh(const rh_mesh_desc* m, const double* uold, int nvar, int twotond
   };
   for (int l = c.levelmin; l <= c.levelmax; ++l) {
     if (c.noct[l] == 0) continue;
-    const long long box = ((long long)c.box_nx[0] << (l - 1)) * ((long long)c.box_nx[1] << (l - 1)) *
-                          ((long long)c.box_nx[2] << (l - 1));
-    c.levels[l].complete_box = (long long)c.noct[l] == box;
     if (c.levels[l].complete_box) continue;
     const long long gbase = (long long)c.ngridmax + nghost;
     // A small level gets shorter pencils so that it still fills a wave of

@@ -57,7 +57,7 @@ struct LevelTables {
 struct Context {
   bool inited = false;
   TileCfg amr_cfg{8, 4, 2, 32};  // tiles of multi-level meshes (coarse-fine kernels)
-  bool amr_cfg_set = false;     // amr_cfg chosen by rh_set_amr_tile (else by precision at rh_set_mesh)
+  bool amr_cfg_set = false;     // amr_cfg chosen by rh_set_amr_tile (else by choose_amr_tile at rh_set_mesh)
   int table_builder = 1;        // coarse-fine tables: 1 on the device, 0 on the host
   int state_check = 0;          // rh_coarse_step checks every level after set_uold (rh_set_state_check)
   int deterministic = 0;        // FP64 coarse-fine update through face slots (rh_set_deterministic)
@@ -215,6 +215,8 @@ int ensure_level_tables(int l);
 TileCfg level_cfg(int l);  // tile of level l's launches (see rh_api.cu)
 // rh_tile.cu: tile and depth of a uniform level of nxo x nyo x nzo octs
 TileCfg choose_tile(int precision, int nxo, int nyo, int nzo, int sm_count);
+// ... and of a mesh of several levels (complete_box of its levels is set)
+TileCfg choose_amr_tile(const Context& c);
 // rh_hoststep.cu: releases the overlapped host-step schedule (mesh change, finalize)
 void free_host_schedule();
 #ifdef __CUDACC__

@@ -1,4 +1,5 @@
-// rh_tile.cu — the tile a uniform level takes when its user chose none.
+// rh_tile.cu — the tiles a mesh's levels take when their user chose none: a
+// uniform level's here, those of coarse-fine levels at the end.
 //
 // A CTA marches its pencil layer by layer, so a level's step takes the CTAs'
 // waves times a pencil's march: a 64^3 level cut into 8x8-octs x 32-layer
@@ -17,6 +18,7 @@
 // 2.40).  On 25 boxes no choice was slower than 8x8 octs x 32 layers for slope
 // types 0, 1 or 3.
 #include <algorithm>
+#include <vector>
 
 #include "rh_internal.h"
 
@@ -64,6 +66,55 @@ TileCfg choose_tile(int precision, int nxo, int nyo, int nzo, int sm_count) {
     }
   }
   return best;
+}
+
+namespace {
+
+// Layers of the TX x TY tiles that hold an oct of level l: what its pencils
+// march through.  Counted in a bitmap over (tile, layer), hashed where the
+// level's box is larger than 16 bits an oct (a few per cent of the layers may share
+// a bit then, as many with either tile).
+template <int TX, int TY> long long occupied_layers(const Context& c, int l) {
+  const long long nx = (long long)c.box_nx[0] << (l - 1), ny = (long long)c.box_nx[1] << (l - 1),
+                  nz = (long long)c.box_nx[2] << (l - 1);
+  const long long ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY;
+  if (c.levels[l].complete_box) return ntx * nty * nz;
+  int bits = 12;
+  while (bits < 30 && (1ll << bits) < 16ll * c.noct[l]) ++bits;
+  const bool dense = (double)ntx * nty * nz <= (double)(1ll << bits);
+  std::vector<uint64_t> seen((size_t)1 << (bits - 6), 0);
+  long long n = 0;
+  const rh_oct* o = c.grid.data() + (c.head[l] - 1);
+  for (int i = 0; i < c.noct[l]; ++i) {
+    const long long x = o[i].ckey[0], y = o[i].ckey[1], z = o[i].ckey[2];
+    if (x < 0 || y < 0 || z < 0 || x >= nx || y >= ny || z >= nz) continue;  // refused by the table builder
+    uint64_t k = (uint64_t)((y / TY * ntx + x / TX) * nz + z);
+    if (!dense) k = k * 0x9E3779B97F4A7C15ull >> (64 - bits);
+    const uint64_t bit = 1ull << (k & 63);
+    n += !(seen[k >> 6] & bit);
+    seen[k >> 6] |= bit;
+  }
+  return n;
+}
+
+}  // namespace
+
+// Tile of the coarse-fine kernels (levels, boxes and oct records of the mesh
+// set).  FP64: 7x11, whose layer costs least per oct column, unless the mesh
+// fills so few of its columns that the layers of 8x4 tiles, two CTAs an SM, cost
+// less.  The cost ratio follows the measured one: gradient-refined blasts 0.94 to
+// 1.01 by layers, 0.86 to 0.98 measured (levels 6-9: 508 against 549 us a coarse
+// step), a sheet 0.89 and 0.92, scattered clusters of 27 to 343 octs 1.14 to 1.36
+// and 1.17 to 1.29 (levels 6-8: 394 against 311 us; a third fewer ghost octs too).
+TileCfg choose_amr_tile(const Context& c) {
+  if (c.precision == RH_PREC_FP32_BULK) return TileCfg{7, 7, 2, 32};
+  double wide = 0, narrow = 0;
+  for (int l = c.levelmin; l <= c.levelmax; ++l) {
+    if (c.noct[l] == 0) continue;
+    wide += 7.04 * occupied_layers<7, 11>(c, l);
+    narrow += 0.5 * 6.95 * occupied_layers<8, 4>(c, l);
+  }
+  return wide > 1.04 * narrow ? TileCfg{8, 4, 2, 32} : TileCfg{7, 11, 1, 32};
 }
 
 }  // namespace rh

@@ -10,7 +10,7 @@ import pytest
 from ramses2_b200._abi import HydroParams
 from ramses2_b200.batch import Batch, ic_blast, problem
 from ramses2_b200.hydro import GodunovGPU
-from ramses2_b200.mesh import prim_to_cons, sedov_amr_mesh, uniform_mesh
+from ramses2_b200.mesh import amr_mesh, fill_amr_prim, prim_to_cons, sedov_amr_mesh, uniform_mesh
 
 pytestmark = pytest.mark.gpu
 
@@ -141,3 +141,44 @@ def test_totals_and_the_neighbours(prec, tile):
         assert list(sa["totals"]) == list(sb["totals"])
     else:  # another order of 98,304 positive terms
         assert sa["totals"] == pytest.approx(sb["totals"], rel=1e-13)
+
+
+def scattered(lmin, lmax, every, nexpand):
+    """Clusters of (2 nexpand + 1)^3 octs around every so many-th cell."""
+    def refine(x, l):
+        k = (x * 2 ** l).astype(np.int64)
+        return ((k[:, 0] * 73856093) ^ (k[:, 1] * 19349663) ^ (k[:, 2] * 83492791)) % every == 0
+
+    m = amr_mesh(lmin, lmax, refine, nexpand=nexpand)
+    r = np.random.default_rng(2)
+    fill_amr_prim(m, lambda x, l: (r.uniform(0.5, 1.5, x.shape[:-1]), *r.uniform(-0.3, 0.3, (3,) + x.shape[:-1]),
+                                   r.uniform(0.5, 1.5, x.shape[:-1])), 1.4)
+    return m
+
+
+@pytest.mark.parametrize("which,tile", [("scattered", (8, 4, 2, 32)), ("a few clusters", (7, 11, 1, 32)),
+                                        ("blast", (7, 11, 1, 32))])
+def test_fp64_coarse_fine_tile_by_how_full_its_columns_are(which, tile):
+    """The chosen tile shows in the partial levels' pencils and ghost octs; the
+    states equal those of either tile bit for bit.  (The few clusters in a large
+    box are counted in a hashed bitmap, the others in a dense one.)"""
+    m = {"scattered": lambda: scattered(6, 8, 4001, 2), "a few clusters": lambda: scattered(7, 8, 400001, 2),
+         "blast": lambda: sedov_amr_mesh(6, 8, radius=0.16)[0]}[which]()
+    P = HydroParams.make(gamma=1.4, interpol_type=1)
+    dt = 0.1 * m.dx(m.levelmax)
+    partial = [l for l in range(m.levelmin + 1, m.levelmax + 1) if m.noct[l]]
+    got = []
+    for t in (None, tile, (7, 11, 1, 32) if tile[0] == 8 else (8, 4, 2, 32)):
+        g = GodunovGPU(m, P, precision="fp64", amr_tile=t)
+        try:
+            n = C.c_int()
+            cut = []
+            for l in partial:
+                assert g.L.rh_level_info(l, C.byref(n), None) == 0
+                cut.append((n.value, g.L.rh_level_ghosts(l, None, None, None, 0)))
+            got.append((cut, [g.coarse_step(dt), g.coarse_step()], g.fetch_uold()))
+        finally:
+            g.close()
+    assert got[0][0] == got[1][0] != got[2][0]
+    for other in got[1:]:
+        assert got[0][1] == other[1] and np.array_equal(got[0][2], other[2])
