@@ -77,8 +77,8 @@ int rh_batch_fetch(int id, double* host_uold);
 /* Tile of the batch kernel (one of the compiled shapes rh_batch_list_tiles
  * returns; lz = oct layers per pencil).  Until it is called the tile follows
  * the problems in the batch: 8x4 octs, 2 CTAs per SM, 32 layers (FP32-bulk
- * batches of mostly 2D problems: 7x7), fewer layers where that leaves CTA slots
- * without work. */
+ * batches of mostly 2D problems: 7x7), fewer layers where few problems share
+ * the CTA slots better so. */
 int rh_batch_set_tile(int txo, int tyo, int minb, int lz);
 /* Compiled batch-kernel shapes of a precision: writes up to max entries,
  * returns how many exist. */

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <vector>
 
 #include "ramses_hydro_batch.h"
@@ -367,6 +368,46 @@ TileCfg default_tile(const std::vector<int>& ids) {
   return TileCfg{8, 4, 2, 32};
 }
 
+// Modelled time of a step (us) of n work items, taken in their order by the CTA
+// slots as they get free: an item of L layers takes 9.2 + L * layer, a slot's
+// first one 5.2 more, with one CTA or two on an SM (the layers' rates of
+// rh_tile.cu), one of a 2D problem about 25 us.  On nineteen batches of 16^3 to
+// 160^3 in both precisions (8x4 tile) the depth it picks is within 3 % of the best
+// one, 0.2 % on average.  least: the items' sum over the slots.
+double modelled_step(const std::vector<int>& ids, const std::vector<BatchProb>& probs, long long n, double* least) {
+  Batch& b = B();
+  const int sm = ctx().sm_count;
+  const size_t slots = (size_t)std::max(1, b.cfg.minb) * sm;
+  const bool bulk = b.precision == RH_PREC_FP32_BULK, wide = b.cfg.txo == 7;
+  const double start = 9.2, first = 5.2;
+  const double layer = n <= sm ? (bulk ? (wide ? 3.12 : 2.92) : 5.62) : (bulk ? (wide ? 4.93 : 3.78) : 6.95);
+  std::vector<double> free_at;  // a heap of the slots' ends, the earliest on top
+  free_at.reserve(slots);
+  double end = 0, sum = 0;
+  for (int i : ids) {
+    const BatchProb& P = probs[i];
+    const int nzo = P.ncz / 2;
+    const bool plane = b.plane2d && P.ndim == 2 && nzo == 1 && P.periodic[2];
+    for (int z = 0; z < P.tz; ++z) {
+      const double t = plane ? 25.0 : start + layer * std::min(b.lz, nzo - z * b.lz);
+      for (long long k = 0; k < (long long)P.tx * P.ty; ++k) {
+        if (free_at.size() < slots) {
+          free_at.push_back(first + t);
+          if (free_at.size() == slots) std::make_heap(free_at.begin(), free_at.end(), std::greater<double>());
+          end = std::max(end, first + t);
+        } else {
+          std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
+          end = std::max(end, free_at.back() += t);
+          std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+        }
+        sum += t;
+      }
+    }
+  }
+  *least = first + sum / slots;
+  return end;
+}
+
 // Rebuild the work list (largest problems first) and the step graph.
 int rebuild() {
   Batch& b = B();
@@ -378,22 +419,41 @@ int rebuild() {
   std::sort(ids.begin(), ids.end(), [&](int x, int y) { return b.probs[x].noct > b.probs[y].noct; });
   std::vector<long long> woff(ids.size() + 1, 0);
   std::vector<BatchProb> probs(b.cap);
-  // Pencil depth: the tile's, halved (down to 2) while the batch does not make
-  // a work item for every CTA slot: a few small problems are a few deep pencils,
-  // each marched by one CTA while the others idle (12 FP64 problems of 16^3 to
-  // 64^3: 0.247 -> 0.187 ms a step).  States, times and dt do
-  // not depend on it (a cell's update does not depend on where pencils end, the
-  // dt is a minimum); the conserved totals are summed in another order.
+  // Pencil depth: the tile's, or a halved one (down to 2) where the modelled step
+  // is shorter by 2 % or more: a few problems are a few deep pencils, marched by
+  // one CTA each while other slots idle or wait for the last of them (FP64: three
+  // of 64^3 215 -> 136 us, one of 144^3 462 -> 374), while shallower ones march
+  // more halo layers (140 of 16^3, one wave at 8 layers: 78 us, 87 with 4).  From
+  // eight items a slot on the tile's depth is taken: the last wave is a small
+  // part.  States, times and dt do not depend on it (a cell's update does not
+  // depend on where pencils end, the dt is a minimum); the conserved totals are
+  // summed in another order.
   if (!b.cfg_set) b.cfg = default_tile(ids);
   const long long slots = (long long)std::max(1, b.cfg.minb) * c.sm_count;
-  b.lz = b.cfg.lz;
-  for (;; b.lz /= 2) {
+  auto cut = [&](int lz) {
+    b.lz = lz;
     long long work = 0;
     for (int i : ids) {
       probs[i] = make_prob(b.probs[i].p, b.probs[i].oct0);
       work += (long long)probs[i].tx * probs[i].ty * probs[i].tz;
     }
-    if (b.cfg_set || b.lz <= 2 || work >= slots) break;
+    return work;
+  };
+  long long work = cut(b.cfg.lz);
+  if (!b.cfg_set && work < 8 * slots) {
+    double least, best = modelled_step(ids, probs, work, &least);
+    int pick = b.lz;
+    for (int lz = b.cfg.lz / 2; lz >= 2; lz /= 2) {
+      work = cut(lz);
+      if (work >= 8 * slots) break;
+      const double t = modelled_step(ids, probs, work, &least);
+      if (least > best) break;  // shallower ones only add halo layers
+      if (t < 0.98 * best) {
+        best = t;
+        pick = lz;
+      }
+    }
+    if (pick != b.lz) cut(pick);
   }
   for (size_t s = 0; s < ids.size(); ++s) {
     const BatchProb& P = probs[ids[s]];
