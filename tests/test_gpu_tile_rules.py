@@ -182,3 +182,31 @@ def test_fp64_coarse_fine_tile_by_how_full_its_columns_are(which, tile):
     assert got[0][0] == got[1][0] != got[2][0]
     for other in got[1:]:
         assert got[0][1] == other[1] and np.array_equal(got[0][2], other[2])
+
+
+# fewer items than SMs, than slots, a few more than slots, several a slot; 3D and with a 2D problem
+BATCHES = [[(32, 32, 32)] * 3, [(96, 96, 96)], [(16, 16, 16)] * 100, [(32, 32, 32)] * 40,
+           [(128, 32, 64)] * 6 + [(256, 256, 2)], [(48, 80, 72), (16, 16, 128), (96, 64, 32)]]
+
+
+@pytest.mark.parametrize("sizes", BATCHES)
+@pytest.mark.parametrize("prec", ["fp64", "fp32_bulk"])
+def test_default_depth_of_few_and_of_many_work_items(prec, sizes):
+    got = []
+    for tile in (None, (8, 4, 2, 32)):
+        b = Batch(prec, pool_octs=sum(n[0] * n[1] * n[2] // 8 for n in sizes) + 8, tile=tile)
+        try:
+            ids = []
+            for k, n in enumerate(sizes):
+                plane = n[2] == 2
+                ids.append(b.add(problem(n, dx=1 / 32, ndim=2 if plane else 3, max_steps=3 + k % 2,
+                                         bc=["outflow"] * 4 + ["periodic"] * 2 if plane else "reflexive"),
+                                 ic_blast([1.0, 0.1, 0.05 * (k % 5), 0.0, 0.1], 5.0, 0.1, [0.3, 0.2, 0.03])))
+            b.step(4)
+            got.append([(b.status(i), b.fetch(i)) for i in (ids[0], ids[len(ids) // 2], ids[-1])])
+        finally:
+            b.close()
+    for (sa, ua), (sb, ub) in zip(*got):
+        assert (sa["t"], sa["dt"], sa["nstep"]) == (sb["t"], sb["dt"], sb["nstep"])
+        assert sa["totals"] == pytest.approx(sb["totals"], rel=1e-12)
+        assert np.array_equal(ua, ub)
