@@ -18,6 +18,7 @@
 // 2.40).  On 25 boxes no choice was slower than 8x8 octs x 32 layers for slope
 // types 0, 1 or 3.
 #include <algorithm>
+#include <new>
 #include <vector>
 
 #include "rh_internal.h"
@@ -109,10 +110,14 @@ template <int TX, int TY> long long occupied_layers(const Context& c, int l) {
 TileCfg choose_amr_tile(const Context& c) {
   if (c.precision == RH_PREC_FP32_BULK) return TileCfg{7, 7, 2, 32};
   double wide = 0, narrow = 0;
-  for (int l = c.levelmin; l <= c.levelmax; ++l) {
-    if (c.noct[l] == 0) continue;
-    wide += 7.04 * occupied_layers<7, 11>(c, l);
-    narrow += 0.5 * 6.95 * occupied_layers<8, 4>(c, l);
+  try {
+    for (int l = c.levelmin; l <= c.levelmax; ++l) {
+      if (c.noct[l] == 0) continue;
+      wide += 7.04 * occupied_layers<7, 11>(c, l);
+      narrow += 0.5 * 6.95 * occupied_layers<8, 4>(c, l);
+    }
+  } catch (const std::bad_alloc&) {  // no room to count in (128 MB at most)
+    return TileCfg{7, 11, 1, 32};
   }
   return wide > 1.04 * narrow ? TileCfg{8, 4, 2, 32} : TileCfg{7, 11, 1, 32};
 }
